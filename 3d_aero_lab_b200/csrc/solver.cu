@@ -761,7 +761,12 @@ extern "C" int a3d_solver_write(a3d_solver* s, const float* r, const float* ru, 
 // per plane but keep the SMs busy and the z chunks of a3d_solver_step overlapping.  Measured
 // (G cell-updates/s, fighter): 15.8M cells 32 planes 16.0 (16: 15.7); 4.1M 16 planes 15.1 (32:
 // 13.8); 2.0M 8 planes 13.5 (16: 12.2); 1.0M 4 planes 12.6 (8: 11.8); 0.3M 2 planes 7.3 (8:
-// 5.6); 31k 2 planes 1.5 (8: 0.7).  Not part of the reference surface.
+// 5.6); 31k 2 planes 1.5 (8: 0.7).
+// The paired tile takes single planes where all of them fit the chip at once: the stage is then
+// one CTA's latency, and a plane less in it counts for more than the planes read twice (us per
+// iteration, 1 plane against 2: 20k cells 16.4 / 24.1, 31k 17.9 / 24.6, 98k, 258 of 296 resident
+// CTAs, 20.5 / 24.6; beyond one wave it turns, 150k, 396 CTAs, 32.8 / 28.7).
+// Not part of the reference surface.
 extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t march_kz) {
   clear_error();
   A3D_ARG(s, "null solver");
@@ -779,6 +784,7 @@ extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t marc
       auto ctas = [&](int kz) { return columns * ((s->grid.NZ + kz - 1) / kz); };
       march_kz = 2;
       if (ctas(32) >= 4L * resident) march_kz = 32;
+      else if (kernel == KERNEL_PAIR && ctas(1) <= resident) march_kz = 1;
       else
         for (int kz : {16, 8, 4})
           if (ctas(kz) >= 2L * resident) { march_kz = kz; break; }

@@ -186,8 +186,8 @@ int a3d_solver_interp_state(a3d_solver* fine, const a3d_solver* coarse);
  *           in packed f32x2 arithmetic, two CTAs per SM.
  * (Numbers 1 and 3 belonged to two tiles since retired; they are refused.)
  * march_kz = z planes per thread block; 0 (the default) picks for the TMA tiles 32 planes if
- * that still launches four waves of CTAs, else the longest of 16, 8 or 4 planes that
- * launches two waves, else 2.                                                            */
+ * that still launches four waves of CTAs, else (kernel 4) single planes if all their CTAs are
+ * resident at once, else the longest of 16, 8 or 4 planes that launches two waves, else 2. */
 int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t march_kz);
 int a3d_solver_get_kernel(a3d_solver* s, int32_t* kernel, int32_t* march_kz);
 /* Bounded device waits; no counterpart in the reference.  Every wait of a stage kernel (the

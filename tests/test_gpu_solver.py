@@ -134,6 +134,22 @@ def test_pipelined_z_chunks_are_bit_identical(aero, chunks, kernel):
     assert a.residual(1) == b.residual(1)
 
 
+@pytest.mark.parametrize("cells,kz", [(2000, 1), (98000, 1), (150000, 2)])
+def test_automatic_z_run_takes_single_planes_on_one_wave(aero, cells, kz):
+    """Kernel 4's automatic z run: single planes where all their CTAs are resident at once, longer
+    runs beyond; the state is the 16-plane run's within the tile's z-run rounding (4e-6)."""
+    sh = aero.shape_of(aero.build_aircraft("interceptor" if cells == 98000 else "airliner"))
+    _, a = gpu_case(aero, sh, cells, 1.0, kernel=4)
+    _, b = gpu_case(aero, sh, cells, 1.0, kernel=4)
+    assert a.kernel() == (4, kz)
+    b.set_kernel(4, 16)
+    for s in (a, b):
+        s.set_chunks(1)
+        s.step(20)
+    A, B = a.read_array(), b.read_array()
+    assert max(rel_max_diff(A[c], B[c]) for c in range(5)) < 4e-6
+
+
 @pytest.mark.parametrize("kernel", [2, 4])
 def test_bounded_wait_runs_out_reports_timeout_and_recovers(aero, kernel):
     """The TMA tiles' bounded waits (SURVEY failure detection): with the wait limit at 0 every wait
