@@ -45,7 +45,7 @@ constexpr double kDeg = kPi / 180;                   // src/field.js:7
 // far-field and symmetry-mirror ghost cells of a tile.
 enum : uint8_t { T_FLUID = 0, T_SOLID = 1, T_SINK = 3, T_JETB = 4, T_JETC = 5, T_GHOST = 6, T_MIRROR = 7 };
 // Code byte: bits 0-2 type, bit 3/4/5 MUSCL slope allowed in x/y/z (static part of the
-// test at src/air_cfd.js:214), bit 6 "irregular" (phi != 1 or a +face aperture != 1),
+// test at src/air_cfd.js:214), bit 6 "irregular" (phi or one of its six faces' apertures != 1),
 // bit 7 "baffle" (this cell's or the lower cell's +z face carries a baffle slope).
 enum : uint8_t { C_OKX = 8, C_OKY = 16, C_OKZ = 32, C_IRR = 64, C_BAF = 128 };
 

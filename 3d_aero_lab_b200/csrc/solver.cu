@@ -44,7 +44,9 @@ __global__ void k_codes(int NX, int NY, int NZ, int NXp, const uint8_t* t, const
       if (j > 0 && j + 1 < NY && fluid(q - NX) && fluid(q + NX) && ap1[q - NX] == 1.f && ap1[q] == 1.f) c |= C_OKY;
       if (k > 0 && k + 1 < NZ && fluid(q - NXY) && fluid(q + NXY) && ap2[q - NXY] == 1.f && ap2[q] == 1.f) c |= C_OKZ;
     }
-    if (phi[q] != 1.f || ap0[q] != 1.f || ap1[q] != 1.f || ap2[q] != 1.f) c |= C_IRR;
+    if (phi[q] != 1.f || ap0[q] != 1.f || ap1[q] != 1.f || ap2[q] != 1.f || (i > 0 && ap0[q - 1] != 1.f) ||
+        (j > 0 && ap1[q - NX] != 1.f) || (k > 0 && ap2[q - NXY] != 1.f))
+      c |= C_IRR;
     if (ap3[q] != 0.f || (k > 0 && ap3[q - NXY] != 0.f)) c |= C_BAF;
     code[((long)k * NY + j) * NXp + i] = c;
   }

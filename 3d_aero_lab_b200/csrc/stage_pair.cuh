@@ -9,6 +9,14 @@
 //   * residual, local time step, RK update and clamps of the two cells: packed.
 // Every face is evaluated once per tile; the tile's +x and +y edge faces by two warps.
 //
+// What bounds it: instruction issue with four warps per scheduler (128 registers), so the plane
+// loop is kept short and what only cells beside a body need - apertures, the wall-pressure
+// source, baffles - stands behind one test of the pair's codes.  9009 warp instructions per plane
+// of a tile in stage 1 (9712 with the apertures carried through shared memory and the wall term
+// formed for every cell); fighter 4.13M cells 17.05 -> 18.7 G cell-updates/s, airliner 120M 19.9 ->
+// 22.3.  The loop must also fit the instruction caches: unrolled by two planes, which removes the
+// 42 register moves a plane and pair, it is 37 KB long and measured 18.0 at 120M.
+//
 // The planes arrive through a 4-deep ring of shared-memory slots filled by
 // `cp.async.bulk.tensor` (one 40 x 20 x 5-component state box and one 64 x 20 code box per
 // plane, completing on the slot's mbarrier; no cluster multicast).  Per plane k:
@@ -58,9 +66,7 @@ struct PairSmem {
   float2 P[5][HY][NP];          // plane-k primitives; pair p holds cells (i0-2+2p, i0-1+2p)
   uint16_t C[HY][NP];           // their codes, first cell in the low byte
   float2 Fx[5][TY][TX / 2 + 1]; // a * flux of x faces (x0-1/2, x0+1/2) of each pair; [16].x: the +x edge face
-  float2 Ax[TY][TX / 2 + 1];
   float2 Fy[5][TY + 1][TX / 2]; // a * flux of the y faces j-1/2 of each pair; row TY: the +y edge faces
-  float2 Ay[TY + 1][TX / 2];
   uint64_t bar[NSLOT];
   int abort;
 };
@@ -141,11 +147,22 @@ __device__ __forceinline__ uint32_t slot_pair(const StageArgs& a, const Slot& s,
   return e0 | (e1 << 8);
 }
 
+// Fluxes of two cells' +faces times their apertures, where the codes say that one may differ from 1.
+__device__ __forceinline__ void weigh(uint32_t c, const float* ap, int q, f2 G[5]) {
+  if (c & (C_IRR | C_IRR << 8)) {
+    f2 A = f2s(1.f);
+    if (c & C_IRR) A.x = __ldg(ap + q);
+    if (c & (C_IRR << 8)) A.y = __ldg(ap + q + 1);
+#pragma unroll
+    for (int v = 0; v < 5; v++) G[v] = mul(A, G[v]);
+  }
+}
+
 // x faces x0-1/2 (lane x) and x0+1/2 (lane y) of the cell pair at plane-array pair p, row y
 // (cells x0, x0+1 of row jj, plane k).  c: the pair's primitives; cl, cc: codes of the pair to
 // the left and of this pair.  The slopes of cells x0-1, x0, x0+1 are each formed once.
-// G: aperture-weighted fluxes (mass, x-, y-, z-momentum, energy); returns the apertures.
-__device__ __forceinline__ f2 xfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cl,
+// G: aperture-weighted fluxes (mass, x-, y-, z-momentum, energy).
+__device__ __forceinline__ void xfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cl,
                                      uint32_t cc, int q, uint32_t okm, f2 G[5]) {
   const float h1 = half_if((cl >> 8) & okm, C_OKX), h2 = half_if(cc & okm, C_OKX);
   const float h3 = half_if((cc >> 8) & okm, C_OKX);
@@ -161,21 +178,21 @@ __device__ __forceinline__ f2 xfaces(const StageArgs& a, const PairSmem& S, int 
   }
   // face x0-1/2 is cell x0-1's +x face, face x0+1/2 cell x0's (src/air_cfd.js:211, 223-224)
   // q: geometry index of cell x0; a cell outside the domain carries a ghost code, never C_IRR
-  f2 A = f2s(1.f);
-  if ((cl >> 8) & C_IRR) A.x = __ldg(a.ap0 + q - 1);
-  if (cc & C_IRR) A.y = __ldg(a.ap0 + q);
   // a closed face (A = 0) contributes A * F = 0: the flux of its finite states is formed
-  // anyway, without a branch (src/air_cfd.js:223-224 skips it)
-  f2 F[5];
-  hllc2(PP{Ls[0], Ls[1], Ls[2], Ls[3], Ls[4]}, PP{Rs[0], Rs[1], Rs[2], Rs[3], Rs[4]}, F);
+  // anyway (src/air_cfd.js:223-224 skips it)
+  hllc2(PP{Ls[0], Ls[1], Ls[2], Ls[3], Ls[4]}, PP{Rs[0], Rs[1], Rs[2], Rs[3], Rs[4]}, G);
+  if ((cl & (C_IRR << 8)) | (cc & C_IRR)) {
+    f2 A = f2s(1.f);
+    if (cl & (C_IRR << 8)) A.x = __ldg(a.ap0 + q - 1);
+    if (cc & C_IRR) A.y = __ldg(a.ap0 + q);
 #pragma unroll
-  for (int v = 0; v < 5; v++) G[v] = mul(A, F[v]);
-  return A;
+    for (int v = 0; v < 5; v++) G[v] = mul(A, G[v]);
+  }
 }
 
 // y faces j-1/2 of the two cells (x0, x0+1) at plane-array pair p, row y (cell row jj, plane
 // k).  c: their primitives; cb, cc: codes of the pair in row y-1 and of this pair.
-__device__ __forceinline__ f2 yfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cb,
+__device__ __forceinline__ void yfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cb,
                                      uint32_t cc, int qb, uint32_t okm, f2 G[5]) {
   const f2 hL = make_float2(half_if(cb & okm, C_OKY), half_if(cb & okm, C_OKY << 8));
   const f2 hR = make_float2(-half_if(cc & okm, C_OKY), -half_if(cc & okm, C_OKY << 8));
@@ -191,20 +208,17 @@ __device__ __forceinline__ f2 yfaces(const StageArgs& a, const PairSmem& S, int 
   }
   // face j-1/2 is cell (x, j-1)'s +y face; below y = 0 lies the symmetry mirror (open)
   // qb: geometry index of cell (x0, jj-1); ghost and mirror codes never carry C_IRR
-  f2 A = f2s(1.f);
-  if (cb & C_IRR) A.x = __ldg(a.ap1 + qb);
-  if (cb & (C_IRR << 8)) A.y = __ldg(a.ap1 + qb + 1);
-  f2 F[5];  // closed faces: A * F = 0, no branch
+  f2 F[5];
   hllc2(PP{Ls[0], Ls[2], Ls[1], Ls[3], Ls[4]}, PP{Rs[0], Rs[2], Rs[1], Rs[3], Rs[4]}, F);
-  G[0] = mul(A, F[0]); G[1] = mul(A, F[2]); G[2] = mul(A, F[1]); G[3] = mul(A, F[3]); G[4] = mul(A, F[4]);
-  return A;
+  G[0] = F[0]; G[1] = F[2]; G[2] = F[1]; G[3] = F[3]; G[4] = F[4];
+  weigh(cb, a.ap1, qb, G);
 }
 
 // z faces k+1/2 of the pair: cells b (plane k, primitives Pb, codes cb) and c (plane k+1, Pc,
 // cc), with e (plane k+2, Pe) above.  Lb is b's +z face state, carried from the face below;
 // c's slope gives this face's right state and, in Lc, the left state of the face above: each
 // z slope is formed once.  qb: geometry index of b's first cell.
-__device__ __forceinline__ f2 zfaces(const StageArgs& a, const f2 Lb[5], const f2 Pb[5], const f2 Pc[5],
+__device__ __forceinline__ void zfaces(const StageArgs& a, const f2 Lb[5], const f2 Pb[5], const f2 Pc[5],
                                      const f2 Pe[5], uint32_t cb, uint32_t cc, int qb, uint32_t okm, f2 G[5],
                                      f2 Lc[5]) {
   const f2 h = make_float2(half_if(cc & okm, C_OKZ), half_if(cc & okm, C_OKZ << 8));
@@ -218,26 +232,62 @@ __device__ __forceinline__ f2 zfaces(const StageArgs& a, const f2 Lb[5], const f
     Lc[v] = fma(h, s, Pc[v]);
   }
   // cells outside the domain carry ghost codes, never C_IRR
-  f2 A = f2s(1.f);
-  if (cb & C_IRR) A.x = __ldg(a.ap2 + qb);
-  if (cb & (C_IRR << 8)) A.y = __ldg(a.ap2 + qb + 1);
-  f2 F[5];  // closed faces: A * F = 0, no branch
+  f2 F[5];
   hllc2(PP{Lb[0], Lb[3], Lb[1], Lb[2], Lb[4]}, PP{Rc[0], Rc[3], Rc[1], Rc[2], Rc[4]}, F);
-  G[0] = mul(A, F[0]); G[1] = mul(A, F[2]); G[2] = mul(A, F[3]); G[3] = mul(A, F[1]); G[4] = mul(A, F[4]);
-  return A;
+  G[0] = F[0]; G[1] = F[2]; G[2] = F[3]; G[3] = F[1]; G[4] = F[4];
+  weigh(cb, a.ap2, qb, G);
 }
 
-// Baffle transpiration of one cell (src/air_cfd.js:226-233): w = u dz/dx through the +z face
-// (slope sUp = ap3 of the cell) and the -z face (sDn = ap3 of the cell below), with the cell's
-// own state; Am, Ap: the cell's -z and +z apertures.
-__device__ __forceinline__ void baffle(const StageArgs& a, int q, int k, int NXY, float r, float u, float v, float w,
-                                       float pC, float Am, float Ap, float rz, float R[5]) {
-  const float sUp = __ldg(a.ap3 + q), sDn = k > 0 ? __ldg(a.ap3 + q - NXY) : 0.f;
-  if (sUp != 0.f || sDn != 0.f) {
-    const float Hh = (pC / kGm + 0.5f * r * (u * u + v * v + w * w) + pC) / r;
-    const float m = (sDn != 0.f ? (1.f - Am) * r * u * sDn : 0.f) - (sUp != 0.f ? (1.f - Ap) * r * u * sUp : 0.f);
-    const float mh = m * rz;
-    R[0] += mh; R[1] += mh * u; R[2] += mh * v; R[3] += mh * w; R[4] += mh * Hh;
+// What only cells beside a body have: the wall-pressure source of faces partly closed, the
+// transpiration of a baffle and the division by the volume fraction ph (cells x0, x0 + 1 of row j,
+// plane k, of primitives r .. p and codes c).
+__device__ __forceinline__ void irregular(const StageArgs& a, uint32_t c, int x0, int j, int k, f2 rx, f2 ry, f2 rz,
+                                       f2 r, f2 u, f2 v, f2 w, f2 p, f2 ph, f2 R[5]) {
+  const long NXY = (long)a.NX * a.NY, q0 = k * NXY + (long)j * a.NX + x0;
+  f2 dA[3];  // + face aperture less - face aperture
+  f2 Az[2] = {f2s(1.f), f2s(1.f)};
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    float ax0 = 1.f, ax1 = 1.f, ay0 = 1.f, ay1 = 1.f, az0 = 1.f, az1 = 1.f;
+    const long q = q0 + e;
+    if ((c >> (8 * e)) & C_IRR) {  // beyond the domain, and below y = 0 (the symmetry plane), faces are open
+      ax1 = __ldg(a.ap0 + q);
+      ay1 = __ldg(a.ap1 + q);
+      az1 = __ldg(a.ap2 + q);
+      if (x0 + e > 0) ax0 = __ldg(a.ap0 + q - 1);
+      if (j > 0) ay0 = __ldg(a.ap1 + q - a.NX);
+      if (k > 0) az0 = __ldg(a.ap2 + q - NXY);
+    }
+    (e ? dA[0].y : dA[0].x) = ax1 - ax0;
+    (e ? dA[1].y : dA[1].x) = ay1 - ay0;
+    (e ? dA[2].y : dA[2].x) = az1 - az0;
+    (e ? Az[0].y : Az[0].x) = az0;
+    (e ? Az[1].y : Az[1].x) = az1;
+  }
+  // wall-pressure source (src/air_cfd.js:225)
+  R[1] = fma(mul(p, dA[0]), rx, R[1]);
+  R[2] = fma(mul(p, dA[1]), ry, R[2]);
+  R[3] = fma(mul(p, dA[2]), rz, R[3]);
+  // baffle transpiration (src/air_cfd.js:226-233): w = u dz/dx through the +z face (slope sUp = ap3
+  // of the cell) and the -z face (sDn = ap3 of the cell below), with the cell's own state
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    if (!((c >> (8 * e)) & C_BAF)) continue;
+    const float sUp = __ldg(a.ap3 + q0 + e), sDn = k > 0 ? __ldg(a.ap3 + q0 + e - NXY) : 0.f;
+    if (sUp == 0.f && sDn == 0.f) continue;
+    const float r1 = e ? r.y : r.x, u1 = e ? u.y : u.x, v1 = e ? v.y : v.x, w1 = e ? w.y : w.x, p1 = e ? p.y : p.x;
+    const float Am = e ? Az[0].y : Az[0].x, Ap = e ? Az[1].y : Az[1].x;
+    const float Hh = (p1 / kGm + 0.5f * r1 * (u1 * u1 + v1 * v1 + w1 * w1) + p1) / r1;
+    const float m = (sDn != 0.f ? (1.f - Am) * r1 * u1 * sDn : 0.f) - (sUp != 0.f ? (1.f - Ap) * r1 * u1 * sUp : 0.f);
+    const float mh = m * rz.x;
+    const float add[5] = {1.f, u1, v1, w1, Hh};
+#pragma unroll
+    for (int i = 0; i < 5; i++) (e ? R[i].y : R[i].x) = i ? fmaf(mh, add[i], e ? R[i].y : R[i].x) : (e ? R[0].y : R[0].x) + mh;
+  }
+  if (ph.x != 1.f || ph.y != 1.f) {
+    const f2 iph = make_float2(1.f / ph.x, 1.f / ph.y);
+#pragma unroll
+    for (int i = 0; i < 5; i++) R[i] = mul(R[i], iph);
   }
 }
 
@@ -246,10 +296,13 @@ __device__ __forceinline__ void baffle(const StageArgs& a, int q, int k, int NXY
 template <bool PUSH>
 __device__ __forceinline__ void store_pair(const StageArgs& a, float* __restrict__ Out, long qp, int k, bool in1,
                                            const f2 o[5]) {
+  float* p = Out + qp;
+  if (in1) {
 #pragma unroll
-  for (int c = 0; c < 5; c++) {
-    if (in1) *reinterpret_cast<float2*>(Out + c * a.Np + qp) = o[c];
-    else Out[c * a.Np + qp] = o[c].x;
+    for (int c = 0; c < 5; c++, p += a.Np) *reinterpret_cast<float2*>(p) = o[c];
+  } else {
+#pragma unroll
+    for (int c = 0; c < 5; c++, p += a.Np) *p = o[c].x;
   }
   if (PUSH) {
 #pragma unroll
@@ -320,7 +373,6 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
 
   bool ok = true;
   f2 W0[5], W1[5], Lz[5], Gz[5];  // column window (planes k, k+1), carried +z state, flux of face k-1/2
-  f2 Az;
   uint32_t c0, c1;
   {
     f2 Wa[5], Wm[5], Lm[5];
@@ -338,7 +390,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
       const f2 d1 = sub(Wm[v], Wa[v]), d2 = sub(W0[v], Wm[v]);
       Lm[v] = fma(hm, make_float2(minmod(d1.x, d2.x), minmod(d1.y, d2.y)), Wm[v]);
     }
-    Az = zfaces(a, Lm, Wm, W0, W1, cm, c0, (k0 - 1) * NXY + q0, okm, Gz, Lz);
+    zfaces(a, Lm, Wm, W0, W1, cm, c0, (k0 - 1) * NXY + q0, okm, Gz, Lz);
   }
   if (!ok) S.abort = 1;
   __syncthreads();  // slots of planes k0-2 and k0-1 are free again
@@ -377,45 +429,45 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
       last_issued = k + 3;
     }
     // ---- [B] x and y face fluxes ----
+    f2 ph = f2s(1.f);  // on its way while the fluxes are formed
+    if (c0 & C_IRR) ph.x = __ldg(a.phi + q);
+    if (c0 & (C_IRR << 8)) ph.y = __ldg(a.phi + q + 1);
     {
       f2 G[5];
-      const f2 A = xfaces(a, S, hy, pp, W0, S.C[hy][pp - 1], c0, q, okm, G);
+      xfaces(a, S, hy, pp, W0, S.C[hy][pp - 1], c0, q, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fx[v][ty][tx2] = G[v];
-      S.Ax[ty][tx2] = A;
     }
     {
       f2 G[5];
-      const f2 A = yfaces(a, S, hy, pp, W0, S.C[hy - 1][pp], c0, q - a.NX, okm, G);
+      yfaces(a, S, hy, pp, W0, S.C[hy - 1][pp], c0, q - a.NX, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fy[v][ty][tx2] = G[v];
-      S.Ay[ty][tx2] = A;
     }
     if (t >= 192 && t < 192 + TX / 2) {  // warp 6: the +y edge faces j0+TY-1/2
       const int e = t - 192;
       f2 c[5], G[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) c[v] = S.P[v][TY + 2][e + 1];
-      const f2 A = yfaces(a, S, TY + 2, e + 1, c, S.C[TY + 1][e + 1], S.C[TY + 2][e + 1],
+      yfaces(a, S, TY + 2, e + 1, c, S.C[TY + 1][e + 1], S.C[TY + 2][e + 1],
                           k * NXY + (j0 + TY - 1) * a.NX + i0 + 2 * e, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fy[v][TY][e] = G[v];
-      S.Ay[TY][e] = A;
     } else if (t >= 224 && t < 224 + TY) {  // warp 7: the +x edge faces i0+TX-1/2, one per row (lane x)
       const int r = t - 224;
       f2 c[5], G[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) c[v] = S.P[v][r + 2][TX / 2 + 1];
-      const f2 A = xfaces(a, S, r + 2, TX / 2 + 1, c, S.C[r + 2][TX / 2], S.C[r + 2][TX / 2 + 1],
+      xfaces(a, S, r + 2, TX / 2 + 1, c, S.C[r + 2][TX / 2], S.C[r + 2][TX / 2 + 1],
                           k * NXY + (j0 + r) * a.NX + i0 + TX, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fx[v][r][TX / 2] = G[v];
-      S.Ax[r][TX / 2] = A;
     }
     f2 bq[5];
     if (STAGE2 && in0) {
+      const float* p = Bp + qp;
 #pragma unroll
-      for (int c = 0; c < 5; c++) bq[c] = __ldg(reinterpret_cast<const float2*>(Bp + c * Np + qp));
+      for (int c = 0; c < 5; c++, p += Np) bq[c] = __ldg(reinterpret_cast<const float2*>(p));
     }
     // ---- plane k+2 into the column window; z face k+1/2 ----
     ok = mbar_wait(&S.bar[sk2], parity_of(k + 2, k0), a.wait_limit);
@@ -424,7 +476,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     if (!ok) S.abort = 1;
     f2 W2[5], Gn[5], Ln[5];
     const uint32_t c2 = own(k + 2, W2);
-    const f2 An = zfaces(a, Lz, W0, W1, W2, c0, c1, q, okm, Gn, Ln);
+    zfaces(a, Lz, W0, W1, W2, c0, c1, q, okm, Gn, Ln);
     __syncthreads();
     if (S.abort) { first_pending = k + 2; break; }  // the wait for plane k+2 ran out
     // ---- [C] residual and RK update ----
@@ -440,32 +492,8 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
         const f2 fym = S.Fy[c][ty][tx2], fyp = S.Fy[c][ty + 1][tx2];
         R[c] = fma(sub(Gz[c], Gn[c]), rz, fma(sub(fym, fyp), ry, mul(sub(fxm, fxp), rx)));
       }
-      {  // wall-pressure source (src/air_cfd.js:225)
-        const f2 axm = S.Ax[ty][tx2];
-        const f2 axp = make_float2(axm.y, S.Ax[ty][tx2 + 1].x);
-        const f2 aym = S.Ay[ty][tx2], ayp = S.Ay[ty + 1][tx2];
-        const f2 pC = W0[4];
-        R[1] = fma(mul(pC, sub(axp, axm)), rx, R[1]);
-        R[2] = fma(mul(pC, sub(ayp, aym)), ry, R[2]);
-        R[3] = fma(mul(pC, sub(An, Az)), rz, R[3]);
-      }
-      if (c0 & (C_BAF | (C_BAF << 8))) {  // baffle transpiration (rare)
-        float Rx[5] = {R[0].x, R[1].x, R[2].x, R[3].x, R[4].x}, Ry[5] = {R[0].y, R[1].y, R[2].y, R[3].y, R[4].y};
-        if (c0 & C_BAF)
-          baffle(a, q, k, NXY, W0[0].x, W0[1].x, W0[2].x, W0[3].x, W0[4].x, Az.x, An.x, rz.x, Rx);
-        if (in1 && (c0 & (C_BAF << 8)))
-          baffle(a, q + 1, k, NXY, W0[0].y, W0[1].y, W0[2].y, W0[3].y, W0[4].y, Az.y, An.y, rz.y, Ry);
-#pragma unroll
-        for (int c = 0; c < 5; c++) R[c] = make_float2(Rx[c], Ry[c]);
-      }
-      f2 ph = f2s(1.f);
-      if (c0 & C_IRR) ph.x = __ldg(a.phi + q);
-      if (in1 && (c0 & (C_IRR << 8))) ph.y = __ldg(a.phi + q + 1);
-      if (ph.x != 1.f || ph.y != 1.f) {
-        const f2 iph = make_float2(1.f / ph.x, 1.f / ph.y);
-#pragma unroll
-        for (int c = 0; c < 5; c++) R[c] = mul(R[c], iph);
-      }
+      if (c0 & (C_IRR | C_IRR << 8 | C_BAF | C_BAF << 8))
+        irregular(a, c0, x0, j, k, rx, ry, rz, W0[0], W0[1], W0[2], W0[3], W0[4], ph, R);
       // local time step from the base state (src/air_cfd.js:243; stage 2 recomputes it from B = Q)
       f2 Pb[5];
       if (STAGE2) prim2(bq, Pb);
@@ -480,7 +508,9 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
       const f2 sw = make_float2(fabsf(Pb[3].x) + as.x, fabsf(Pb[3].y) + as.y);
       const f2 den = fma(sw, rz, fma(sv, ry, mul(su, rx)));
       const f2 num = mul(f2s(a.cfl), mx(ph, f2s(0.25f)));
-      const f2 dt = make_float2(num.x / den.x, num.y / den.y);
+      // (both divisors lie far inside 2^-126 .. 2^126, where the plain approximate quotient is as
+      // accurate as the full-range one: 2 ulp)
+      const f2 dt = make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
       f2 o[5];
 #pragma unroll
       for (int c = 0; c < 5; c++) {
@@ -491,13 +521,13 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
       // positivity clamps (src/air_cfd.js:247-249)
       o[0] = mx(o[0], f2s(1e-4f));
       const f2 k2 = mul(kPkHalf, fma(o[1], o[1], fma(o[2], o[2], mul(o[3], o[3]))));
-      const f2 ke = make_float2(k2.x / o[0].x, k2.y / o[0].y);
+      const f2 ke = make_float2(__fdividef(k2.x, o[0].x), __fdividef(k2.y, o[0].y));
       const f2 pe = mul(kPkGm, sub(o[4], ke));
       if (pe.x < 1e-5f) o[4].x = 1e-5f / kGm + ke.x;
       if (pe.y < 1e-5f) o[4].y = 1e-5f / kGm + ke.y;
       // solid and fixed-state cells (src/air_cfd.js:242): the base state, or the fixed state
-      const uint32_t t0 = c0 & 7, t1 = (c0 >> 8) & 7;
-      if (t0 != T_FLUID || t1 != T_FLUID) {
+      if (c0 & 0x0707) {  // not both fluid
+        const uint32_t t0 = c0 & 7, t1 = (c0 >> 8) & 7;
 #pragma unroll
         for (int c = 0; c < 5; c++) {
           const f2 base = STAGE2 ? bq[c] : *reinterpret_cast<const f2*>(&sl.Q[c][hy][xs]);
@@ -509,7 +539,6 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     }
 #pragma unroll
     for (int c = 0; c < 5; c++) { Gz[c] = Gn[c]; Lz[c] = Ln[c]; W0[c] = W1[c]; W1[c] = W2[c]; }
-    Az = An;
     c0 = c1;
     c1 = c2;
   }

@@ -258,6 +258,50 @@ def test_random_boxes_per_cell(aero, ref, seed, dims, order, kernel):
             assert d < tol, (c, n, d)
 
 
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("kernel", [0, 2, 4])
+def test_lone_partly_closed_faces(aero, ref, d, kernel):
+    """Faces partly closed between cells that are otherwise whole (phi 1): a cell is irregular
+    through its - face as well.  Faces inside a tile, on the tiles' 32 x 16 and 32 x 8 edges, on a z
+    run's edge and on the domain's + boundary; same tolerance as the random boxes."""
+    NX, NY, NZ = 67, 34, 9
+    rng = np.random.default_rng(5)
+    bg = BoxGrid(rng, NX, NY, NZ)
+    t = np.zeros(bg.N, np.uint8)
+    phi = np.ones(bg.N, np.float32)
+    ap = [np.ones(bg.N, np.float32) for _ in range(3)] + [np.zeros(bg.N, np.float32)]
+    for i in (0, 13, 30, 31, 32, 63, NX - 1):
+        for j in (0, 7, 8, 15, 16, NY - 1):
+            for k in (0, 3, 4, NZ - 1):
+                if (i + 2 * j + 3 * k) % 3 == 0:
+                    ap[d][(k * NY + j) * NX + i] = (0.0, 0.4, 0.75)[(i + j + k) % 3]
+    geo = ref.Geom()
+    geo.t, geo.phi, geo.ap = t, phi, ap
+    o = ref.CfdCPU(bg, geo)
+    hgeo = aero.cfd.Geom(bg.N)
+    hgeo.t, hgeo.phi, hgeo.ap = t, phi, ap
+    s = aero.CfdGPU(aero.cfd.Grid(bg.xf, bg.yf, bg.zf), hgeo)
+    s.set_kernel(kernel, 4)
+    F = freestream(0.7, 4.0)
+    for x in (o, s):
+        x.setFree(F)
+        x.setFix([F, F, F])
+        x.reset()
+    Q0 = o.read()
+    noise = rng.standard_normal(Q0.shape)
+    Q0 = Q0 * (1 + 0.05 * noise)
+    Q0[2] += 0.05 * noise[2] * Q0[0]
+    Q0 = Q0.astype(np.float32).astype(np.float64)
+    o.write(Q0)
+    s.write(Q0.astype(np.float32))
+    o.step(1)
+    s.step(1)
+    Qo, Qg = o.read(), s.read_array()
+    for c in range(5):
+        e = float(np.max(np.abs(Qg[c] - Qo[c]) / np.abs(Qo[c]))) if c in (0, 4) else rel_max_diff(Qg[c], Qo[c])
+        assert e < 2e-5, (c, e)
+
+
 def test_postprocessing_matches_oracle(aero, ref):
     ac, sh, og, ogeo, o = oracle_case(aero, ref, "airliner", 150000, 1.0, M=0.78, alpha=2.5)
     g, s = gpu_case(aero, sh, 150000, 1.0, M=0.78, alpha=2.5)
