@@ -100,12 +100,13 @@ struct a3d_solver {
 
 namespace a3d {
 int solver_finish_setup(a3d_solver* s);           // codes + force list + state buffers
-int launch_stage(a3d_solver* s, const StageArgs& a);
+int launch_stage(a3d_solver* s, const StageArgs& a, bool dependent = false);
 void fill_stage_args(a3d_solver* s, StageArgs& a, const float* Qin, const float* B, float* Out, float wa, float wb);
 int build_force_list(a3d_solver* s);
 int make_tensor_maps(a3d_solver* s);
 int launch_tma(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cudaStream_t st = nullptr);
-int launch_pair(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cudaStream_t st = nullptr);
+int launch_pair(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cudaStream_t st = nullptr,
+                bool dependent = false);
 int make_pair_tensor_maps(a3d_solver* s);
 size_t pair_smem_bytes();
 int pair_resident_ctas(int* n);         // CTAs of the paired-tile stage kernel resident on the current device

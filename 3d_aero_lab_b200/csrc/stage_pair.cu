@@ -31,10 +31,20 @@ int set_attributes() {
 }
 
 template <int MODE>
-void launch_mode(const a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, dim3 grid, cudaStream_t st) {
-  const size_t sm = pair_smem_bytes();
-  if (stage2) k_stage_pair<true, MODE><<<grid, NT, sm, st>>>(s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
-  else k_stage_pair<false, MODE><<<grid, NT, sm, st>>>(s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
+void launch_mode(const a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, dim3 grid, cudaStream_t st,
+                 bool dependent) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = pair_smem_bytes();
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  if (stage2) cudaLaunchKernelEx(&cfg, k_stage_pair<true, MODE>, s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
+  else cudaLaunchKernelEx(&cfg, k_stage_pair<false, MODE>, s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
 }
 
 }  // namespace
@@ -85,13 +95,14 @@ int make_pair_tensor_maps(a3d_solver* s) {
 }
 
 // The paired-tile stage kernel over planes [a.kb, a.ke) on stream st (the solver's by default).
-int launch_pair(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cudaStream_t st) {
+// dependent: the launch may start while the stream's previous one is ending.
+int launch_pair(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cudaStream_t st, bool dependent) {
   const int kz = s->march_kz;
   dim3 grid((a.NX + TX - 1) / TX, (a.NY + TY - 1) / TY, (a.ke - a.kb + kz - 1) / kz);
   if (!st) st = s->st;
-  if (a.peer[0] || a.peer[1]) launch_mode<2>(s, a, qin_buf, stage2, grid, st);
-  else if (a.kb != 0 || a.ke != a.NZ) launch_mode<1>(s, a, qin_buf, stage2, grid, st);
-  else launch_mode<0>(s, a, qin_buf, stage2, grid, st);
+  if (a.peer[0] || a.peer[1]) launch_mode<2>(s, a, qin_buf, stage2, grid, st, dependent);
+  else if (a.kb != 0 || a.ke != a.NZ) launch_mode<1>(s, a, qin_buf, stage2, grid, st, dependent);
+  else launch_mode<0>(s, a, qin_buf, stage2, grid, st, dependent);
   A3D_CUDA(cudaGetLastError());
   return A3D_OK;
 }

@@ -361,6 +361,10 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     fence_barrier_init();
   }
   __syncthreads();
+  if (!PERSISTENT && !RANGE) {  // (z chunks and slabs are ordered by events instead)
+    pdl_launch_dependents();
+    pdl_wait();  // the state that the launch before this one wrote
+  }
   if (t == 0) {
     fence_proxy_async_smem();  // earlier tiles' generic reads of the slots before these copies
     for (int p = k0 - 2; p <= k0 + 1; p++) issue_plane(S, tmQ, tmC, a, p, k0, i0, j0);
