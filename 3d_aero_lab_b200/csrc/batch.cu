@@ -372,10 +372,10 @@ extern "C" int a3d_batch_create(a3d_solver* const* solvers, int32_t n, a3d_batch
   b->ev_join.assign(n, nullptr);
   for (int k = 0; k < n && e == cudaSuccess; k++) e = cudaEventCreateWithFlags(&b->ev_join[k], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_cases, (size_t)n * sizeof(BatchCase));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_counters, 8 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = dev_alloc(&b->d_cases, (size_t)n * sizeof(BatchCase));
+  if (e == cudaSuccess) e = dev_alloc(&b->d_counters, 8 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(unsigned long long), b->st);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_err, kErrWords * sizeof(long long));
+  if (e == cudaSuccess) e = dev_alloc(&b->d_err, kErrWords * sizeof(long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_err, 0, kErrWords * sizeof(long long), b->st);
   if (e != cudaSuccess) { set_error("batch setup: %s", cudaGetErrorString(e)); rc = e == cudaErrorMemoryAllocation ? A3D_ERR_NOMEM : A3D_ERR_CUDA; }
   if (rc == A3D_OK) {
@@ -400,9 +400,9 @@ extern "C" int a3d_batch_destroy(a3d_batch* b) {
   cudaSetDevice(b->device);
   if (b->st) cudaStreamSynchronize(b->st);
   free_graph(b);
-  cudaFree(b->d_cases);
-  cudaFree(b->d_counters);
-  cudaFree(b->d_err);
+  dev_free(b->d_cases);
+  dev_free(b->d_counters);
+  dev_free(b->d_err);
   for (cudaEvent_t e : b->ev_in) if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : b->ev_join) if (e) cudaEventDestroy(e);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -490,7 +490,7 @@ extern "C" int a3d_batch_tune(a3d_batch* b, int32_t trial_iters, int32_t* best_k
   for (int k = 0; k < n && rc == A3D_OK; k++) {
     a3d_solver* s = b->solvers[k];
     A3D_CUDA(cudaStreamSynchronize(s->st));
-    if (cudaMalloc(&saved[k], 5 * s->Np * sizeof(float)) != cudaSuccess) { set_error("tune: no memory for the state copy"); rc = A3D_ERR_NOMEM; break; }
+    if (dev_alloc(&saved[k], 5 * s->Np * sizeof(float)) != cudaSuccess) { set_error("tune: no memory for the state copy"); rc = A3D_ERR_NOMEM; break; }
     A3D_CUDA(cudaMemcpyAsync(saved[k], s->buf[s->iQ], 5 * s->Np * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
     saved_it[k] = s->it;
   }
@@ -537,7 +537,8 @@ extern "C" int a3d_batch_tune(a3d_batch* b, int32_t trial_iters, int32_t* best_k
     cudaStreamSynchronize(b->st);
     if (saved[k]) {
       cudaMemcpy(s->buf[s->iQ], saved[k], 5 * s->Np * sizeof(float), cudaMemcpyDeviceToDevice);
-      cudaFree(saved[k]);
+      cudaDeviceSynchronize();
+      dev_free(saved[k]);
     }
     s->it = saved_it[k];
   }

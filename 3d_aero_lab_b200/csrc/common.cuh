@@ -36,6 +36,26 @@ void clear_error();
 // Makes `device` current; A3D_ERR_NODEVICE if no CUDA device is visible.
 int use_device(int device);
 
+// Device memory of the current device from the library's pool (runtime.cu).  dev_alloc / dev_free:
+// like cudaMalloc and cudaFree, but a block is freed only once no work that uses it is queued on
+// any stream (cudaFree would have waited).  temp_alloc: stream-ordered, freed by cudaFreeAsync.
+cudaError_t dev_alloc_raw(void** p, size_t bytes);
+void dev_free(void* p);
+cudaError_t temp_alloc_raw(void** p, size_t bytes, cudaStream_t st);
+template <typename T>
+cudaError_t dev_alloc(T** p, size_t bytes) { return dev_alloc_raw((void**)p, bytes); }
+template <typename T>
+cudaError_t temp_alloc(T** p, size_t bytes, cudaStream_t st) { return temp_alloc_raw((void**)p, bytes, st); }
+// Non-blocking streams of the current device, kept for reuse; put back with no work on them.
+cudaError_t stream_get(cudaStream_t* st);
+void stream_put(cudaStream_t st);
+// Lets device `peer` address the pool of `device` (cudaDeviceEnablePeerAccess does not cover pools).
+cudaError_t pool_peer_access(int device, int peer);
+// A small page-locked block of kPinnedBytes.
+constexpr size_t kPinnedBytes = 64 * sizeof(double);
+cudaError_t pinned_alloc(double** p);
+void pinned_free(double* p);
+
 constexpr double kGamma = 1.4;                       // src/air_cfd.js:11
 constexpr double kPi = 3.141592653589793;
 constexpr double kDeg = kPi / 180;                   // src/field.js:7

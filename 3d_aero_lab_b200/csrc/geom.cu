@@ -267,10 +267,10 @@ int geom_build_device(const a3d_shape& shape, const GridDev& gd, double h, doubl
     rc = e == cudaErrorMemoryAllocation ? A3D_ERR_NOMEM : A3D_ERR_CUDA;
   };
   cudaError_t e;
-  if ((e = cudaMallocAsync(&d_shape, sizeof(a3d_shape), st)) != cudaSuccess) { fail(e, "cudaMallocAsync(shape)"); return rc; }
-  if ((e = cudaMallocAsync(&cin, nodes, st)) != cudaSuccess) fail(e, "cudaMallocAsync(node flags)");
-  if (rc == A3D_OK && (e = cudaMallocAsync(&mark, N, st)) != cudaSuccess) fail(e, "cudaMallocAsync(marks)");
-  if (rc == A3D_OK && (e = cudaMallocAsync(&d_cnt, 2 * sizeof(unsigned long long), st)) != cudaSuccess) fail(e, "cudaMallocAsync(counts)");
+  if ((e = temp_alloc(&d_shape, sizeof(a3d_shape), st)) != cudaSuccess) { fail(e, "device memory (shape)"); return rc; }
+  if ((e = temp_alloc(&cin, nodes, st)) != cudaSuccess) fail(e, "device memory (node flags)");
+  if (rc == A3D_OK && (e = temp_alloc(&mark, N, st)) != cudaSuccess) fail(e, "device memory (marks)");
+  if (rc == A3D_OK && (e = temp_alloc(&d_cnt, 2 * sizeof(unsigned long long), st)) != cudaSuccess) fail(e, "device memory (counts)");
   if (rc == A3D_OK) {
     GeoDev g;
     g.a = d_shape;

@@ -132,7 +132,7 @@ extern "C" int a3d_solver_interp_state(a3d_solver* fine, const a3d_solver* coars
   }
   void* dmap = nullptr;
   const size_t bytes = tot * (sizeof(double) + sizeof(int));
-  A3D_CUDA(cudaMallocAsync(&dmap, bytes, fine->st));
+  A3D_CUDA(temp_alloc(&dmap, bytes, fine->st));
   double* dt = (double*)dmap;
   int* di = (int*)(dt + tot);
   int rc = A3D_OK;

@@ -246,21 +246,21 @@ int build_force_list(a3d_solver* s) {
   FlArgs f = fl_args(s);
   int* d_counts = nullptr;
   long* d_off = nullptr;
-  A3D_CUDA(cudaMalloc(&d_counts, nb * sizeof(int)));
+  A3D_CUDA(dev_alloc(&d_counts, nb * sizeof(int)));
   std::vector<int> counts(nb);
   k_fl_count<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_counts);
   cudaError_t e = cudaMemcpyAsync(counts.data(), d_counts, nb * sizeof(int), cudaMemcpyDeviceToHost, s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
-  if (e != cudaSuccess) { cudaFree(d_counts); set_error("force list count: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
+  if (e != cudaSuccess) { dev_free(d_counts); set_error("force list count: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
   std::vector<long> off(nb);
   long tot = 0;
   for (long b = 0; b < nb; b++) { off[b] = tot; tot += counts[b]; }
   s->fl.n = tot;
   const size_t n1 = (size_t)std::max(tot, 1L);
   char* blk = nullptr;
-  e = cudaMalloc(&blk, n1 * (8 + 4 * 8) + 256);
-  if (e == cudaSuccess) e = cudaMalloc(&d_off, nb * sizeof(long));
-  if (e != cudaSuccess) { cudaFree(d_counts); cudaFree(blk); set_error("force list alloc: %s", cudaGetErrorString(e)); return A3D_ERR_NOMEM; }
+  e = dev_alloc(&blk, n1 * (8 + 4 * 8) + 256);
+  if (e == cudaSuccess) e = dev_alloc(&d_off, nb * sizeof(long));
+  if (e != cudaSuccess) { dev_free(d_counts); dev_free(blk); set_error("force list alloc: %s", cudaGetErrorString(e)); return A3D_ERR_NOMEM; }
   s->fl.block = blk;
   s->fl.q = (int64_t*)blk;
   s->fl.cx = (double*)(blk + n1 * 8);
@@ -272,8 +272,8 @@ int build_force_list(a3d_solver* s) {
     k_fl_write<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_off, s->fl.q, s->fl.cx, s->fl.cz, s->fl.x, s->fl.z);
     e = cudaStreamSynchronize(s->st);
   }
-  cudaFree(d_counts);
-  cudaFree(d_off);
+  dev_free(d_counts);
+  dev_free(d_off);
   if (e != cudaSuccess) { set_error("force list write: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
   return A3D_OK;
 }
@@ -400,7 +400,8 @@ extern "C" int a3d_solver_set_owned(a3d_solver* s, int32_t k0, int32_t k1) {
   A3D_CUDA(cudaStreamSynchronize(s->st));
   s->own_k0 = k0;
   s->own_k1 = k1;
-  if (s->fl.block) cudaFree(s->fl.block);
+  A3D_CUDA(cudaDeviceSynchronize());  // nothing still reads the list
+  dev_free(s->fl.block);
   s->fl = ForceList();
   return build_force_list(s);
 }

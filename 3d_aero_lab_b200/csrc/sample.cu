@@ -112,7 +112,7 @@ extern "C" int a3d_solver_sample(a3d_solver* s, int32_t n, const double* xyz, do
   A3D_CUDA(cudaSetDevice(s->device));
   char* buf = nullptr;
   const size_t bx = (size_t)n * 3 * 8, bo = (size_t)n * 5 * 8, bk = (size_t)n * 4;
-  A3D_CUDA(cudaMallocAsync(&buf, bx + bo + bk, s->st));
+  A3D_CUDA(temp_alloc(&buf, bx + bo + bk, s->st));
   double* dxyz = (double*)buf;
   double* dout = (double*)(buf + bx);
   int* dok = (int*)(buf + bx + bo);

@@ -252,35 +252,59 @@ int launch_stage(a3d_solver* s, const StageArgs& a, bool dependent) {
   return A3D_OK;
 }
 
+namespace {
+
+// Number of pipelined z chunks a3d_solver_step uses: kernels 2 and 4 on a whole case only.  Automatic:
+// four chunks from 0.8M cells up, where a stage takes long enough to hide the extra stream and
+// event calls (measured: 4.1M-cell fighter 13.5 -> 15.1 G cell-updates/s, 1.0M-cell airliner
+// 10.1 -> 11.2), none below (0.6M-cell interceptor 8.4 -> 8.1 with four).
+int chunk_count(const a3d_solver* s) {
+  if ((s->kernel != KERNEL_TMA && s->kernel != KERNEL_PAIR) || s->nbr[0] || s->nbr[1] || s->own_k0 != 0 ||
+      s->own_k1 != s->grid.NZ)
+    return 1;
+  const int runs = (s->grid.NZ + s->march_kz - 1) / s->march_kz;
+  const int K = s->chunks_req > 0 ? s->chunks_req : (s->N >= 800000 ? 4 : 1);
+  return std::max(1, std::min(K, std::min(runs, (int)kMaxChunks)));
+}
+
+// The streams and events of K z chunks.
+int chunk_streams(a3d_solver* s, int K) {
+  if (!s->ev_fork) A3D_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
+  for (int c = 0; c < K; c++) {
+    if (!s->cst[c]) A3D_CUDA(stream_get(&s->cst[c]));
+    for (int t = 0; t < 2; t++)
+      if (!s->cev[c][t]) A3D_CUDA(cudaEventCreateWithFlags(&s->cev[c][t], cudaEventDisableTiming));
+  }
+  return A3D_OK;
+}
+
+}  // namespace
+
 int solver_finish_setup(a3d_solver* s) {
   const long N = s->N;
   s->NXp = (int)round_up(s->grid.NX, 16);
   s->Np = round_up((long)s->NXp * s->grid.NY * s->grid.NZ, 64);
   // the tiled stage kernels index cells and padded cells of one component in 32-bit integers
   A3D_ARG(s->Np < (1L << 31), "grid too large: more than 2^31 padded cells per component");
-  A3D_CUDA(cudaMalloc(&s->state, 3 * 5 * s->Np * sizeof(float)));
+  A3D_CUDA(dev_alloc(&s->state, 3 * 5 * s->Np * sizeof(float)));
   for (int b = 0; b < 3; b++) s->buf[b] = s->state + (long)b * 5 * s->Np;
   A3D_CUDA(cudaMemsetAsync(s->state, 0, 3 * 5 * s->Np * sizeof(float), s->st));
-  A3D_CUDA(cudaMalloc(&s->code, round_up(s->Np, 256)));
+  A3D_CUDA(dev_alloc(&s->code, round_up(s->Np, 256)));
   A3D_CUDA(cudaMemsetAsync(s->code, T_GHOST, round_up(s->Np, 256), s->st));
   k_codes<<<blocks_for(N), 256, 0, s->st>>>(s->grid.NX, s->grid.NY, s->grid.NZ, s->NXp, s->geo.t, s->geo.phi,
                                             s->geo.ap0, s->geo.ap1, s->geo.ap2, s->geo.ap3, s->code);
   A3D_CUDA(cudaGetLastError());
-  A3D_CUDA(cudaMalloc(&s->d_red, 4096 * 8 * sizeof(double)));
-  A3D_CUDA(cudaMallocHost(&s->h_red, 64 * sizeof(double)));
-  A3D_CUDA(cudaMalloc(&s->d_flag, 16));
+  A3D_CUDA(dev_alloc(&s->d_red, 4096 * 8 * sizeof(double)));
+  A3D_CUDA(pinned_alloc(&s->h_red));
+  A3D_CUDA(dev_alloc(&s->d_flag, 16));
   A3D_CUDA(cudaMemsetAsync(s->d_flag, 0, 16, s->st));
-  A3D_CUDA(cudaMalloc(&s->prevR, s->Np * sizeof(float)));
+  A3D_CUDA(dev_alloc(&s->prevR, s->Np * sizeof(float)));
   s->own_k0 = 0;
   s->own_k1 = s->grid.NZ;
-  A3D_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
-  for (int c = 0; c < kMaxChunks; c++) {
-    A3D_CUDA(cudaStreamCreateWithFlags(&s->cst[c], cudaStreamNonBlocking));
-    for (int t = 0; t < 2; t++) A3D_CUDA(cudaEventCreateWithFlags(&s->cev[c][t], cudaEventDisableTiming));
-  }
   A3D_TRY(build_force_list(s));
   A3D_TRY(make_tensor_maps(s));
   A3D_TRY(a3d_solver_set_kernel(s, s->kernel, 0));  // the automatic z run
+  if (chunk_count(s) > 1) A3D_TRY(chunk_streams(s, kMaxChunks));
   const double F0[5] = {1, 0, 0, 0, 1 / (kGamma * (kGamma - 1))};  // src/air_cfd.js:162
   for (int c = 0; c < 5; c++) { s->F[c] = F0[c]; s->fix[0][c] = s->fix[1][c] = s->fix[2][c] = F0[c]; }
   A3D_CUDA(cudaStreamSynchronize(s->st));
@@ -301,13 +325,13 @@ int new_solver(int device, const int32_t dims[3], const double* xf, const double
   A3D_TRY(use_device(device));
   a3d_solver* s = new a3d_solver();
   cudaGetDevice(&s->device);
-  if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
+  if (stream_get(&s->st) != cudaSuccess) {
     delete s;
     set_error("cudaStreamCreate failed");
     return A3D_ERR_CUDA;
   }
   if (cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming) != cudaSuccess) {
-    cudaStreamDestroy(s->st);
+    stream_put(s->st);
     delete s;
     set_error("cudaEventCreate failed");
     return A3D_ERR_CUDA;
@@ -400,24 +424,25 @@ extern "C" int a3d_solver_create_shape_slab(const a3d_shape* shape, const int32_
 extern "C" int a3d_solver_destroy(a3d_solver* s) {
   if (!s) return A3D_OK;
   cudaSetDevice(s->device);
-  if (s->st) cudaStreamSynchronize(s->st);
-  cudaFree(s->state);
-  cudaFree(s->code);
-  cudaFree(s->d_red);
-  if (s->h_red) cudaFreeHost(s->h_red);
-  cudaFree(s->d_flag);
-  cudaFree(s->prevR);
-  if (s->fl.block) cudaFree(s->fl.block);
+  // all work that may use the solver's memory, a caller's on streams of its own included
+  cudaDeviceSynchronize();
+  dev_free(s->state);
+  dev_free(s->code);
+  dev_free(s->d_red);
+  pinned_free(s->h_red);
+  dev_free(s->d_flag);
+  dev_free(s->prevR);
+  dev_free(s->fl.block);
   geom_free(s->geo);
   grid_free(s->grid);
   if (s->ev) cudaEventDestroy(s->ev);
   if (s->ev_fork) cudaEventDestroy(s->ev_fork);
   for (int c = 0; c < kMaxChunks; c++) {
-    if (s->cst[c]) cudaStreamDestroy(s->cst[c]);
+    stream_put(s->cst[c]);
     for (int t = 0; t < 2; t++)
       if (s->cev[c][t]) cudaEventDestroy(s->cev[c][t]);
   }
-  if (s->st) cudaStreamDestroy(s->st);
+  stream_put(s->st);
   delete s;
   return A3D_OK;
 }
@@ -469,19 +494,6 @@ extern "C" int a3d_solver_reset(a3d_solver* s) {
 
 namespace {
 
-// Number of pipelined z chunks a3d_solver_step uses: kernels 2 and 4 on a whole case only.  Automatic:
-// four chunks from 0.8M cells up, where a stage takes long enough to hide the extra stream and
-// event calls (measured: 4.1M-cell fighter 13.5 -> 15.1 G cell-updates/s, 1.0M-cell airliner
-// 10.1 -> 11.2), none below (0.6M-cell interceptor 8.4 -> 8.1 with four).
-int chunk_count(const a3d_solver* s) {
-  if ((s->kernel != KERNEL_TMA && s->kernel != KERNEL_PAIR) || s->nbr[0] || s->nbr[1] || s->own_k0 != 0 ||
-      s->own_k1 != s->grid.NZ)
-    return 1;
-  const int runs = (s->grid.NZ + s->march_kz - 1) / s->march_kz;
-  const int K = s->chunks_req > 0 ? s->chunks_req : (s->N >= 800000 ? 4 : 1);
-  return std::max(1, std::min(K, std::min(runs, kMaxChunks)));
-}
-
 // n iterations with the case cut into K z chunks of whole z runs (so every cell sees the same
 // arithmetic as in one launch).  Chunk c's stage waits for the previous stage of chunks c-1 and
 // c+1 only: a stage reads two planes beyond its chunk and writes inside it, so those are its
@@ -493,6 +505,7 @@ int step_chunked(a3d_solver* s, int n, int K) {
     kb[c] = (c * runs / K) * kz;
     ke[c] = std::min(NZ, ((c + 1) * runs / K) * kz);
   }
+  A3D_TRY(chunk_streams(s, K));  // (there already, unless the caller has set the chunks)
   A3D_CUDA(cudaEventRecord(s->ev_fork, s->st));
   for (int c = 0; c < K; c++) A3D_CUDA(cudaStreamWaitEvent(s->cst[c], s->ev_fork, 0));
   bool first = true;
@@ -627,6 +640,7 @@ extern "C" int a3d_solver_set_neighbors(a3d_solver* s, a3d_solver* lo, a3d_solve
       const cudaError_t e = cudaDeviceEnablePeerAccess(n->device, 0);
       if (e == cudaErrorPeerAccessAlreadyEnabled) cudaGetLastError();
       else A3D_CUDA(e);
+      A3D_CUDA(pool_peer_access(n->device, s->device));
     }
   }
   if (lo) A3D_ARG(lo->z_lo < s->z_lo, "lower neighbour must start below");
@@ -665,6 +679,11 @@ extern "C" int a3d_solver_copy_planes(a3d_solver* dst, int32_t dst_k0, a3d_solve
           "plane range");
   const long plane = (long)src->grid.NY * src->NXp;
   const size_t bytes = (size_t)nk * plane * sizeof(float);
+  if (src->device != dst->device) {  // where the devices are peers, the copy goes straight across
+    pool_peer_access(src->device, dst->device);
+    pool_peer_access(dst->device, src->device);
+    cudaGetLastError();
+  }
   const float* sp = state_buffer(src, which) + src_k0 * plane;
   float* dp = state_buffer(dst, which) + dst_k0 * plane;
   A3D_CUDA(cudaSetDevice(src->device));
@@ -707,7 +726,7 @@ extern "C" int a3d_solver_read_dt(a3d_solver* s, float* dt) {
   A3D_ARG(s->phase == 0, "between the two stages of an iteration");
   A3D_CUDA(cudaSetDevice(s->device));
   float* d = nullptr;
-  A3D_CUDA(cudaMallocAsync(&d, s->N * sizeof(float), s->st));
+  A3D_CUDA(temp_alloc(&d, s->N * sizeof(float), s->st));
   if (s->it == 0) {
     A3D_CUDA(cudaMemsetAsync(d, 0, s->N * sizeof(float), s->st));
   } else {

@@ -341,6 +341,38 @@ def test_nonfinite_state_is_reported(aero):
     assert e.value.status == 4
 
 
+def test_cases_made_and_dropped_by_several_threads_agree(aero):
+    """Solvers take their memory, streams and result blocks from pools that outlive them: threads
+    that make, run and drop cases side by side get the states and forces of a case alone."""
+    import threading
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    sizes = (9000, 30000, 60000, 21000)
+
+    def solve(cells):
+        g, s = gpu_case(aero, sh, cells, 3.0)
+        s.step(12)
+        out = s.read_array(), s.forces(3.0, 0.6, 27.9, 8.5, 0.0, 3.3), s.sample(np.array([[1.0, 0.5, 0.2]]))[0]
+        s.dispose()
+        return out
+
+    alone = [solve(c) for c in sizes]
+    bad = []
+
+    def work(n):
+        for r in range(6):
+            k = (n + r) % len(sizes)
+            Q, f, p = solve(sizes[k])
+            if not (np.array_equal(Q, alone[k][0]) and f == alone[k][1] and np.array_equal(p, alone[k][2])):
+                bad.append((n, r))
+
+    ts = [threading.Thread(target=work, args=(n,)) for n in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
 def test_display_sampling_matches_oracle(aero, ref):
     """cfdStencil + cfdSample on the device vs the oracle, on the same state (FP64 both)."""
     ac, sh, og, ogeo, o = oracle_case(aero, ref, "airliner", 150000, 2.0, M=0.78, alpha=2.5)
