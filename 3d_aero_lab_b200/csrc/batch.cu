@@ -235,12 +235,38 @@ std::vector<double> signature(const a3d_solver* s) {
   return v;
 }
 
+// Mode 1: the z run of the cases whose own is automatic (paired tile only, whose results do not
+// depend on the run), 0 to leave them.  A case's own run is short enough to fill the chip alone;
+// beside others it need not be, and each run costs four planes read and a z face formed twice.
+// So: 16 planes where all cases together still launch two waves of CTAs, else 8 or 4 planes where
+// that makes 1.2 waves.  Measured (us per iteration; own runs, 4, 8, 16 planes): 24 cases, 5.1M
+// cells 475, 408, 372, 369 (3.4 waves at 16); 5 cases, 4.4M 322, 301, 281, 280 (2.4); 8 cases, 2.5M
+// 226, 197, 188, 192 (1.5); 12 cases, 1.5M 156, 131, 128, 141 (1.0); 4 cases, 0.57M 66, 60, 73, 98 (0.5).
+int common_run(a3d_batch* b, int* kz) {
+  *kz = 0;
+  if (b->tma_tile) return A3D_OK;
+  int resident = 0;
+  A3D_TRY(pair_resident_ctas(&resident));
+  for (int run : {16, 8, 4}) {
+    long ctas = 0;
+    for (const a3d_solver* s : b->solvers) {
+      const int r = s->kz_auto ? run : s->march_kz;
+      ctas += (long)((s->grid.NX + pair::TX - 1) / pair::TX) * ((s->grid.NY + pair::TY - 1) / pair::TY) *
+              ((s->grid.NZ + r - 1) / r);
+    }
+    if (ctas * 5 >= (run == 16 ? 10L : 6L) * resident) { *kz = run; break; }
+  }
+  return A3D_OK;
+}
+
 // Mode 1: two iterations of every case with its own stage kernel, captured from its own stream
 // forked off the batch stream, so that the graph's per-case branches run concurrently.  Each
 // case's arithmetic is exactly its single-case step.
 int build_stream_graph(a3d_batch* b) {
   if (b->sgraph) cudaGraphExecDestroy(b->sgraph);
   b->sgraph = nullptr;
+  int kz = 0;
+  A3D_TRY(common_run(b, &kz));
   cudaGraph_t g = nullptr;
   A3D_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
   int rc = A3D_OK;
@@ -250,6 +276,8 @@ int build_stream_graph(a3d_batch* b) {
   cu(cudaEventRecord(b->ev_fork, b->st));
   for (size_t k = 0; k < b->solvers.size() && rc == A3D_OK; k++) {
     a3d_solver* s = b->solvers[k];
+    const int own_kz = s->march_kz;
+    if (kz && s->kz_auto) s->march_kz = kz;
     cu(cudaStreamWaitEvent(s->st, b->ev_fork, 0));
     int iQ = s->iQ, iB = s->iB;
     const int iS1 = s->iS1;
@@ -264,6 +292,7 @@ int build_stream_graph(a3d_batch* b) {
       }
       std::swap(iQ, iB);
     }
+    s->march_kz = own_kz;
     cu(cudaEventRecord(b->ev_join[k], s->st));
     cu(cudaStreamWaitEvent(b->st, b->ev_join[k], 0));
   }

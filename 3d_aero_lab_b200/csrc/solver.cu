@@ -796,6 +796,7 @@ extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t marc
   A3D_ARG(s, "null solver");
   A3D_ARG(kernel == KERNEL_CELL || kernel == KERNEL_TMA || kernel == KERNEL_PAIR, "kernel must be 0, 2 or 4");
   A3D_ARG(march_kz >= 0 && march_kz <= 1024, "march_kz");
+  const bool automatic = march_kz == 0;
   if (march_kz == 0) {
     march_kz = 16;
     if (kernel == KERNEL_TMA || kernel == KERNEL_PAIR) {
@@ -816,6 +817,7 @@ extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t marc
   }
   s->kernel = kernel;
   s->march_kz = march_kz;
+  s->kz_auto = automatic;
   return A3D_OK;
 }
 

@@ -76,6 +76,7 @@ struct a3d_solver {
   CUtensorMap tmCp;
   uint32_t wait_limit = A3D_WAIT_LIMIT_DEFAULT;  // try_waits a stage kernel spends on one TMA copy
   int march_kz = 16;              // z planes per CTA of the marching kernels
+  bool kz_auto = true;            // picked from the grid size, not by the caller
   // reductions
   double* d_red = nullptr;        // device partials + results
   double* h_red = nullptr;        // pinned host mirror of the results

@@ -81,6 +81,28 @@ def test_stream_mode_equals_individual_steps(aero, n):
     b.dispose()
 
 
+@pytest.mark.parametrize("scale", [0.1, 1, 4, 14])
+def test_automatic_z_runs_in_a_batch_leave_the_results(aero, scale):
+    """Mode 1 over the paired tile: cases whose z run is automatic share a longer one (none, 4, 8 and
+    16 planes at these sizes), a case with a run of its own keeps it; every state is the case's alone."""
+    def cases():
+        out = [aero.Case(aircraft_type=c[0], cells=c[1] * scale, M=c[2], alpha=c[3], delta=c[4]) for c in CASES]
+        out[1].solver.set_kernel(4, 5)
+        return out
+
+    alone, batched = cases(), cases()
+    b = aero.Batch([c.solver for c in batched])
+    for n in (4, 3):
+        for c in alone:
+            c.solver.step(n)
+        b.step(n)
+        b.sync()
+        for a, c in zip(alone, batched):
+            assert c.solver.kernel() == a.solver.kernel()
+            assert np.array_equal(c.solver.read_array(), a.solver.read_array())
+    b.dispose()
+
+
 def test_tma_tile_z_run_changes_only_rounding(aero):
     """The TMA tile with z runs of 8 and 64 planes: the same solution to float32 rounding."""
     a, b = make(aero, 2, *CASES[1]), make(aero, 2, *CASES[1])
