@@ -295,6 +295,7 @@ int solver_finish_setup(a3d_solver* s) {
                                             s->geo.ap0, s->geo.ap1, s->geo.ap2, s->geo.ap3, s->code);
   A3D_CUDA(cudaGetLastError());
   A3D_CUDA(dev_alloc(&s->d_red, 4096 * 8 * sizeof(double)));
+  A3D_CUDA(cudaMemsetAsync(s->d_red, 0, 4096 * 8 * sizeof(double), s->st));
   A3D_CUDA(pinned_alloc(&s->h_red));
   A3D_CUDA(dev_alloc(&s->d_flag, 16));
   A3D_CUDA(cudaMemsetAsync(s->d_flag, 0, 16, s->st));

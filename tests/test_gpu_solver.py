@@ -325,6 +325,25 @@ def test_postprocessing_matches_oracle(aero, ref):
     assert math.isclose(s.residual(3), o.residual(3), rel_tol=1e-9)
 
 
+@pytest.mark.parametrize("cells", [8000, 70000, 1500000])
+def test_residual_strides_and_snapshots(aero, cells):
+    """One pass samples every stride-th fluid cell and takes the next call's snapshot, from less than
+    one turn of the grid to several: the same FP64 terms as numpy's, added in another order."""
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    g, s = gpu_case(aero, sh, cells, 0.0)
+    t = aero.cfd_geom(sh, g, 0.0).t
+    assert s.residual(1) is None
+    was = s.read_array()[0].astype(np.float64).ravel()
+    for n, stride in enumerate((1, 3, 7, g.NX, 997), 1):
+        s.step(n)
+        now = s.read_array()[0].astype(np.float64).ravel()
+        pick = (np.arange(now.size) % stride == 0) & (t.ravel() == 0)
+        want = math.sqrt(np.sum((now - was)[pick] ** 2) / pick.sum()) / n
+        assert math.isclose(s.residual(stride), want, rel_tol=1e-11), stride
+        assert s.residual(stride) is None  # no step since: a snapshot only
+        was = now
+
+
 def test_nonfinite_state_is_reported(aero):
     sh = aero.shape_of(aero.build_aircraft("fighter"))
     g, s = gpu_case(aero, sh, 8000, 0.0)
