@@ -9,6 +9,13 @@
 //   and intake layers -> face clean-up next to solids -> forced-open fixed-cell faces.
 // Results are bit-identical to the reference's arithmetic wherever the device's double
 // transcendentals round like the host's; the tests compare every cell.
+//
+// What bounds a build is latency, not its 21 bytes a cell: the inside tests' FP64 chains in the
+// few cells that the surface cuts, launches and waits.  So the cut cells' samples are spread over
+// their block, the engine layers are marked without the host, and everything that one cell's
+// finished faces need is one pass.  (A 1M-cell airliner case from grid to free stream, with the
+// force list and the codes: 700 us before, 372 us now.)
+#include <algorithm>
 #include <cmath>
 #include <vector>
 #include "geom.cuh"
@@ -75,7 +82,8 @@ __device__ bool solid_at(const GeoDev& g, double x, double y, double z) {
     const double r = (double)v.env_R[k] + ((double)v.env_R[k + 1] - (double)v.env_R[k]) * (f - k);
     if (hypot(ay - v.y, z - v.z) < r) return true;
   }
-  if (x >= 0 && x <= a.fus_L) {  // fuselage (AirGeom.inFus)
+  // fuselage (AirGeom.inFus); no radius exceeds the larger of R0 and Re while noseP >= 0
+  if (x >= 0 && x <= a.fus_L && (ay <= 1.0001 * fmax(a.fus_R0, a.fus_Re) || a.fus_noseP < 0)) {
     const double R = fus_radius(a, x), dz = z - fus_center(a, x);
     if (ay * ay + dz * dz <= R * R) return true;
   }
@@ -99,48 +107,72 @@ __global__ void k_nodes(GeoDev g, uint8_t* cin) {
   }
 }
 
-// phi by 27 sub-samples and the three +face apertures by 9 sub-samples (src/air_cfd.js:73-90).
-__global__ void k_cells(GeoDev g, const uint8_t* cin, float* phi, float* ap0, float* ap1, float* ap2, float* ap3) {
+// phi by 27 sub-samples, the three +face apertures by 9 sub-samples (src/air_cfd.js:73-90) and the
+// solid test (src/air_cfd.js:114).  A block's 8 warps take 32 consecutive cells each, from 8 parts
+// of the grid, so that the cut cells (a few per cent, side by side along the surface) are shared
+// out; the block then takes the samples of its cut cells and faces one a thread.  One thread for
+// all samples of its cell took 100-160 us for 1M cells of an airliner, this takes 31.
+__global__ void __launch_bounds__(256) k_cells(GeoDev g, const uint8_t* __restrict__ cin, float* phi, float* ap0,
+                                               float* ap1, float* ap2, float* ap3, uint8_t* t) {
+  __shared__ uint16_t cut[256], face[3 * 256];  // thread; thread * 3 + direction
+  __shared__ int n_cut, n_face, open[256][4];   // samples outside: of phi, of the +x, +y, +z face
+  __shared__ int ijk[256][3];
   const long NX = g.NX, NY = g.NY, N = NX * NY * g.NZ;
   const long NX1 = NX + 1, NXY1 = NX1 * (NY + 1);
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(q % NX), j = (int)((q / NX) % NY), k = (int)(q / (NX * NY));
-    auto cn = [&](int a, int b, int c) { return (int)cin[c * NXY1 + b * NX1 + a]; };
-    const double xf = g.Xf[i], yf = g.Yf[j], zf = g.Zf[k];
-    const double xd = g.Xd[i], yd = g.Yd[j], zd = g.Zd[k];
-    int s = 0;
-    for (int c = 0; c < 8; c++) s += cn(i + (c & 1), j + ((c >> 1) & 1), k + (c >> 2));
-    float ph;
-    if (s == 0) ph = 1.f;
-    else if (s == 8) ph = 0.f;
-    else {
-      int n = 0;
-      for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++)
-          for (int c = 0; c < 3; c++)
-            if (!solid_at(g, xf + kSub[a] * xd, yf + kSub[b] * yd, zf + kSub[c] * zd)) n++;
-      ph = (float)(n / 27.0);
+  const long tiles = (N + 255) / 256;
+  const int tid = threadIdx.x;
+  for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long q = ((tid >> 5) * tiles + tile) * 32 + (tid & 31);
+    if (tid == 0) n_cut = n_face = 0;
+    for (int w = 0; w < 4; w++) open[tid][w] = 0;
+    __syncthreads();
+    int s = 0, m[3] = {0, 0, 0};
+    if (q < N) {
+      const long row = q / NX;
+      const int i = (int)(q - row * NX), k = (int)(row / NY), j = (int)(row - k * NY);
+      ijk[tid][0] = i; ijk[tid][1] = j; ijk[tid][2] = k;
+      const uint8_t* c = cin + k * NXY1 + j * NX1 + i;
+      const int c000 = c[0], c100 = c[1], c010 = c[NX1], c110 = c[NX1 + 1];
+      const int c001 = c[NXY1], c101 = c[NXY1 + 1], c011 = c[NXY1 + NX1], c111 = c[NXY1 + NX1 + 1];
+      s = c000 + c100 + c010 + c110 + c001 + c101 + c011 + c111;
+      m[0] = c100 + c110 + c101 + c111;
+      m[1] = c010 + c110 + c011 + c111;
+      m[2] = c001 + c101 + c011 + c111;
+      if (s != 0 && s != 8) cut[atomicAdd(&n_cut, 1)] = (uint16_t)tid;
+      for (int d = 0; d < 3; d++)
+        if (m[d] != 0 && m[d] != 4) face[atomicAdd(&n_face, 1)] = (uint16_t)(tid * 3 + d);
     }
-    phi[q] = ph;
-    float apv[3];
-    for (int d = 0; d < 3; d++) {
-      int m;
-      if (d == 0) m = cn(i + 1, j, k) + cn(i + 1, j + 1, k) + cn(i + 1, j, k + 1) + cn(i + 1, j + 1, k + 1);
-      else if (d == 1) m = cn(i, j + 1, k) + cn(i + 1, j + 1, k) + cn(i, j + 1, k + 1) + cn(i + 1, j + 1, k + 1);
-      else m = cn(i, j, k + 1) + cn(i + 1, j, k + 1) + cn(i, j + 1, k + 1) + cn(i + 1, j + 1, k + 1);
-      if (m == 0) { apv[d] = 1.f; continue; }
-      if (m == 4) { apv[d] = 0.f; continue; }
-      int n = 0;
-      for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) {
-          const double x = d == 0 ? g.Xf[i + 1] : xf + kSub[a] * xd;
-          const double y = d == 1 ? g.Yf[j + 1] : yf + (d == 0 ? kSub[a] : kSub[b]) * yd;
-          const double z = d == 2 ? g.Zf[k + 1] : zf + kSub[b] * zd;
-          if (!solid_at(g, x, y, z)) n++;
-        }
-      apv[d] = (float)(n / 9.0);
+    __syncthreads();
+    const int cuts = 27 * n_cut, samples = cuts + 9 * n_face;
+    for (int u = tid; u < samples; u += 256) {
+      int c, d, a, b, e;  // cell (its thread), direction of the face or -1, sample numbers along x, y, z
+      if (u < cuts) {
+        c = cut[u / 27]; d = -1;
+        const int r = u % 27;
+        a = r / 9; b = r / 3 % 3; e = r % 3;
+      } else {
+        const int f = face[(u - cuts) / 9], r = (u - cuts) % 9;
+        c = f / 3; d = f - 3 * c;
+        a = r / 3; b = d == 0 ? r / 3 : r % 3; e = r % 3;
+      }
+      const int i = ijk[c][0], j = ijk[c][1], k = ijk[c][2];
+      double x = g.Xf[i] + kSub[a] * (double)g.Xd[i], y = g.Yf[j] + kSub[b] * (double)g.Yd[j],
+             z = g.Zf[k] + kSub[e] * (double)g.Zd[k];
+      if (d == 0) x = g.Xf[i + 1];
+      if (d == 1) y = g.Yf[j + 1];
+      if (d == 2) z = g.Zf[k + 1];
+      if (!solid_at(g, x, y, z)) atomicAdd(&open[c][d + 1], 1);
     }
-    ap0[q] = apv[0]; ap1[q] = apv[1]; ap2[q] = apv[2]; ap3[q] = 0.f;
+    __syncthreads();
+    if (q < N) {
+      const float ph = s == 0 ? 1.f : s == 8 ? 0.f : (float)(open[tid][0] / 27.0);
+      float ap[3];
+      for (int d = 0; d < 3; d++) ap[d] = m[d] == 0 ? 1.f : m[d] == 4 ? 0.f : (float)(open[tid][d + 1] / 9.0);
+      phi[q] = ph;
+      ap0[q] = ap[0]; ap1[q] = ap[1]; ap2[q] = ap[2]; ap3[q] = 0.f;
+      t[q] = ph < 0.2 ? T_SOLID : T_FLUID;
+    }
+    __syncthreads();  // (the lists and counts are used again)
   }
 }
 
@@ -154,96 +186,156 @@ __device__ bool camber_z(const a3d_surface& S, double sA, double x, double ay, d
   return true;
 }
 
-// Baffle on the z face nearest the mean camber surface of column (i, j): the face aperture
-// is reduced by the planform coverage and the local slope dz/dx is stored in ap3
-// (src/air_cfd.js:94-111).  One thread per column; columns never share a cell.
-__global__ void k_baffle(GeoDev g, int which, float* ap2, float* ap3) {
-  const a3d_surface& S = which == 0 ? g.a->wing : g.a->htail;
-  const double sA = S.sA;
-  const bool rot = which == 1;
-  const long NX = g.NX, NY = g.NY;
-  for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < NX * NY; n += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(n % NX), j = (int)(n / NX);
-    if (g.Yf[j] > S.semi || g.Yf[j + 1] < sA) continue;
-    int cov = 0;
-    double zs = 0, ss = 0;
-    for (int a = 0; a < 3; a++)
-      for (int b = 0; b < 3; b++) {
-        const double x = g.Xf[i] + kSub[a] * (double)g.Xd[i], y = g.Yf[j] + kSub[b] * (double)g.Yd[j];
-        double zm, z1, z0;
-        if (!camber_z(S, sA, x, y, zm)) continue;
-        const double e = 0.02 * s_chord(S, fmin(y, S.semi));
-        const bool ok1 = camber_z(S, sA, x + e, y, z1), ok0 = camber_z(S, sA, x - e, y, z0);
-        double sl = (ok1 && ok0) ? (z1 - z0) / (2 * e) : ok1 ? (z1 - zm) / e : ok0 ? (zm - z0) / e : 0;
-        if (rot) { zm -= (x - g.hp0) * g.tdR; sl -= g.tdR; }
-        cov++; zs += zm; ss += sl;
+// Baffle on the z face nearest the mean camber surface of column (i, j), of the wing and then of
+// the tail: the face aperture is reduced by the planform coverage and the local slope dz/dx is
+// stored in ap3 (src/air_cfd.js:94-111).  Nine lanes per column, one a sample; the first one sums
+// them in the reference's order.  Columns never share a cell.  One thread a column and one launch
+// a surface took 2 x 16 us at 1M cells, this takes 9.
+__global__ void __launch_bounds__(256) k_baffle(GeoDev g, float* ap2, float* ap3) {
+  const long NX = g.NX, columns = NX * g.NY;
+  const int lane = threadIdx.x & 31, r = lane % 9, lead = lane - r;
+  const long warps = (long)gridDim.x * (blockDim.x / 32);
+  for (long w = blockIdx.x * (long)(blockDim.x / 32) + threadIdx.x / 32; 3 * w < columns; w += warps) {
+    const long n = 3 * w + lane / 9;
+    const bool mine = lane < 27 && n < columns;
+    const int i = mine ? (int)(n % NX) : 0, j = mine ? (int)(n / NX) : 0;
+    for (int which = 0; which < 2; which++) {
+      const a3d_surface& S = which == 0 ? g.a->wing : g.a->htail;
+      const double sA = S.sA;
+      double zm = 0, sl = 0;
+      bool hit = false;
+      if (mine && !(g.Yf[j] > S.semi || g.Yf[j + 1] < sA)) {
+        const double x = g.Xf[i] + kSub[r / 3] * (double)g.Xd[i], y = g.Yf[j] + kSub[r % 3] * (double)g.Yd[j];
+        double z1, z0;
+        hit = camber_z(S, sA, x, y, zm);
+        if (hit) {
+          const double e = 0.02 * s_chord(S, fmin(y, S.semi));
+          const bool ok1 = camber_z(S, sA, x + e, y, z1), ok0 = camber_z(S, sA, x - e, y, z0);
+          sl = (ok1 && ok0) ? (z1 - z0) / (2 * e) : ok1 ? (z1 - zm) / e : ok0 ? (zm - z0) / e : 0;
+          if (which == 1) { zm -= (x - g.hp0) * g.tdR; sl -= g.tdR; }
+        }
       }
-    if (!cov) continue;
-    const double zm = zs / cov;
-    int k = 0;
-    while (k < g.NZ - 2 && (double)g.Zc[k + 1] <= zm) k++;
-    const long q = ((long)k * NY + j) * NX + i;
-    ap2[q] = (float)fmin((double)ap2[q], 1 - cov / 9.0);
-    ap3[q] = (float)(ss / cov);
-  }
-}
-
-__global__ void k_solid(long N, const float* phi, uint8_t* t) {  // src/air_cfd.js:114
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x)
-    t[q] = phi[q] < 0.2 ? T_SOLID : T_FLUID;
-}
-
-// One fixed-state layer at x index i: cells whose centre lies in the ring [rin - pad, rout + pad]
-// around the engine axis become type `ty` with phi = 1 (src/air_cfd.js:123, 128).
-__global__ void k_mark(GeoDev g, int i, double ey, double ez, double rin, double rout, int ty, uint8_t bit,
-                       uint8_t* t, float* phi, uint8_t* mark, unsigned long long* count) {
-  const long NY = g.NY, NZ = g.NZ;
-  for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < NY * NZ; n += (long)gridDim.x * blockDim.x) {
-    const int j = (int)(n % NY), k = (int)(n / NY);
-    const double r = hypot((double)g.Yc[j] - ey, (double)g.Zc[k] - ez);
-    if (r <= rout && r >= rin) {
-      const long q = ((long)k * NY + j) * g.NX + i;
-      t[q] = (uint8_t)ty; phi[q] = 1.f; mark[q] |= bit;
-      atomicAdd(count, 1ULL);
+      const unsigned hits = __ballot_sync(0xffffffffu, hit);
+      if (!hits) continue;
+      int cov = 0;
+      double zs = 0, ss = 0;
+      for (int o = 0; o < 9; o++) {
+        const int from = min(lead + o, 31);
+        const double zo = __shfl_sync(0xffffffffu, zm, from), so = __shfl_sync(0xffffffffu, sl, from);
+        if (hits >> from & 1) { cov++; zs += zo; ss += so; }
+      }
+      if (!mine) cov = 0;
+      // first k with a centre above the surface: nine candidates a turn
+      const double zmean = zs / cov;
+      int k = -1;
+      for (int kb = 0; __any_sync(0xffffffffu, cov != 0 && k < 0); kb += 9) {
+        const bool stop = !(kb + r < g.NZ - 2 && (double)g.Zc[kb + r + 1] <= zmean);
+        const unsigned stops = __ballot_sync(0xffffffffu, stop) >> lead & 0x1ffu;
+        if (k < 0 && stops) k = min(kb + __ffs(stops) - 1, max(g.NZ - 2, 0));
+      }
+      if (cov && r == 0) {
+        const long q = ((long)k * g.NY + j) * NX + i;
+        ap2[q] = (float)fmin((double)ap2[q], 1 - cov / 9.0);
+        ap3[q] = (float)(ss / cov);
+      }
     }
   }
 }
 
-// Apertures of faces touching a solid closed; baffle slope dropped on domain-top faces,
-// on closed faces and around fixed cells (src/air_cfd.js:132-136).
-__global__ void k_cleanup(int NX, int NY, int NZ, const uint8_t* t, float* ap0, float* ap1, float* ap2, float* ap3) {
+// Fixed-state layers: cells of one x layer i whose centre lies in the ring [rin, rout] around an
+// engine axis become type `ty` with phi = 1 (src/air_cfd.js:123, 128); a layer that catches no
+// cell centre is marked with a padded ring instead (src/air_cfd.js:124, 129).
+struct Ring {
+  int i, ty;
+  uint8_t bit;
+  double ey, ez, rin, rout, rin_pad, rout_pad;
+};
+struct Rings {
+  static constexpr int kMax = A3D_MAX_ENGINES * (A3D_MAX_EXITS + 1);
+  int n;
+  Ring r[kMax];
+};
+
+// Bit x of *caught: ring x catches a cell centre.
+__global__ void k_ring_caught(GeoDev g, Rings rings, unsigned* caught) {
+  const long NY = g.NY, NZ = g.NZ;
+  unsigned got = 0;
+  for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < NY * NZ; n += (long)gridDim.x * blockDim.x) {
+    const int j = (int)(n % NY), k = (int)(n / NY);
+    for (int x = 0; x < rings.n; x++) {
+      const double r = hypot((double)g.Yc[j] - rings.r[x].ey, (double)g.Zc[k] - rings.r[x].ez);
+      if (r <= rings.r[x].rout && r >= rings.r[x].rin) got |= 1u << x;
+    }
+  }
+  if (got) atomicOr(caught, got);
+}
+
+// One thread marks a (j, k) column of all rings, in the reference's engine and exit order.
+__global__ void k_mark(GeoDev g, Rings rings, const unsigned* caught, uint8_t* t, float* phi, uint8_t* mark) {
+  const long NY = g.NY, NZ = g.NZ;
+  const unsigned got = *caught;
+  for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < NY * NZ; n += (long)gridDim.x * blockDim.x) {
+    const int j = (int)(n % NY), k = (int)(n / NY);
+    for (int x = 0; x < rings.n; x++) {
+      const Ring& R = rings.r[x];
+      const bool pad = !(got >> x & 1);
+      const double r = hypot((double)g.Yc[j] - R.ey, (double)g.Zc[k] - R.ez);
+      if (r <= (pad ? R.rout_pad : R.rout) && r >= (pad ? R.rin_pad : R.rin)) {
+        const long q = ((long)k * NY + j) * g.NX + R.i;
+        t[q] = (uint8_t)R.ty; phi[q] = 1.f; mark[q] |= R.bit;
+      }
+    }
+  }
+}
+
+// A cell's finished faces, from the final types:
+//   apertures of faces touching a solid closed; baffle slope dropped on domain-top faces, on
+//   closed faces and around fixed cells (src/air_cfd.js:132-136);
+//   jet cells open their +x face toward fluid, intake cells the -x neighbour's +x face
+//   (src/air_cfd.js:138; the flat index q +- 1 is used as the reference does);
+//   and the numbers of solid and of cut cells (src/air_cfd.js:139).
+// Two passes and a counting one with two atomics a warp took 50 us for 1M cells, this takes 18.
+__global__ void __launch_bounds__(256) k_finish(int NX, int NY, int NZ, const uint8_t* __restrict__ t,
+                                                const float* __restrict__ phi, const uint8_t* __restrict__ mark,
+                                                float* ap0, float* ap1, float* ap2, float* ap3,
+                                                unsigned long long* out) {
   const long NXY = (long)NX * NY, N = NXY * NZ;
+  unsigned ns = 0, nc = 0;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(q % NX), j = (int)((q / NX) % NY), k = (int)(q / NXY);
-    const bool tq = t[q] == T_SOLID;
-    if (i + 1 < NX && (tq || t[q + 1] == T_SOLID)) ap0[q] = 0.f;
-    if (j + 1 < NY && (tq || t[q + NX] == T_SOLID)) ap1[q] = 0.f;
-    if (k + 1 >= NZ) ap3[q] = 0.f;
-    else if (tq || t[q + NXY] == T_SOLID) { ap2[q] = 0.f; ap3[q] = 0.f; }
-    if (t[q] >= T_SINK || (k + 1 < NZ && t[q + NXY] >= T_SINK)) ap3[q] = 0.f;
+    const long row = q / NX;
+    const int i = (int)(q - row * NX), k = (int)(row / NY), j = (int)(row - (long)k * NY);
+    const uint8_t tq = t[q], tx = q + 1 < N ? t[q + 1] : (uint8_t)T_GHOST;
+    const bool solid = tq == T_SOLID;
+    const float p0 = ap0[q], p1 = ap1[q], p2 = ap2[q], p3 = ap3[q];
+    float a0 = p0, a1 = p1, a2 = p2, a3 = p3;
+    if (i + 1 < NX && (solid || tx == T_SOLID)) a0 = 0.f;
+    if (j + 1 < NY && (solid || t[q + NX] == T_SOLID)) a1 = 0.f;
+    if (k + 1 >= NZ) a3 = 0.f;
+    else {
+      const uint8_t tz = t[q + NXY];
+      if (solid || tz == T_SOLID) { a2 = 0.f; a3 = 0.f; }
+      if (tz >= T_SINK) a3 = 0.f;
+    }
+    if (tq >= T_SINK) a3 = 0.f;
+    if (q + 1 < N && (((mark[q] & 1) && tx == T_FLUID) || ((mark[q + 1] & 2) && tq == T_FLUID))) a0 = 1.f;
+    if (a0 != p0) ap0[q] = a0;
+    if (a1 != p1) ap1[q] = a1;
+    if (a2 != p2) ap2[q] = a2;
+    if (a3 != p3) ap3[q] = a3;
+    if (solid) ns++;
+    else if (tq == T_FLUID && (phi[q] < 1.f || a0 < 1.f || a1 < 1.f || a2 < 1.f)) nc++;
   }
-}
-
-// Jet cells open their +x face toward fluid; intake cells open the -x neighbour's +x face
-// (src/air_cfd.js:138).  The flat index q +- 1 is used as the reference does.
-__global__ void k_force_open(long N, const uint8_t* t, const uint8_t* mark, float* ap0) {
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const uint8_t m = mark[q];
-    if (!m) continue;
-    if ((m & 1) && q + 1 < N && t[q + 1] == T_FLUID) ap0[q] = 1.f;
-    if ((m & 2) && q >= 1 && t[q - 1] == T_FLUID) ap0[q - 1] = 1.f;
+  __shared__ unsigned long long sum[2];
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  ns = __reduce_add_sync(0xffffffffu, ns);
+  nc = __reduce_add_sync(0xffffffffu, nc);
+  if ((threadIdx.x & 31) == 0) {
+    if (ns) atomicAdd(&sum[0], (unsigned long long)ns);
+    if (nc) atomicAdd(&sum[1], (unsigned long long)nc);
   }
-}
-
-__global__ void k_counts(long N, const uint8_t* t, const float* phi, const float* ap0, const float* ap1,
-                         const float* ap2, unsigned long long* out) {  // src/air_cfd.js:139
-  unsigned long long ns = 0, nc = 0;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    if (t[q] == T_SOLID) ns++;
-    else if (t[q] == T_FLUID && (phi[q] < 1.f || ap0[q] < 1.f || ap1[q] < 1.f || ap2[q] < 1.f)) nc++;
-  }
-  for (int o = 16; o; o >>= 1) { ns += __shfl_down_sync(0xffffffffu, ns, o); nc += __shfl_down_sync(0xffffffffu, nc, o); }
-  if ((threadIdx.x & 31) == 0) { atomicAdd(out, ns); atomicAdd(out + 1, nc); }
+  __syncthreads();
+  if (threadIdx.x < 2 && sum[threadIdx.x]) atomicAdd(out + threadIdx.x, sum[threadIdx.x]);
 }
 
 int grid_blocks(long work, int threads = 256) {
@@ -270,7 +362,7 @@ int geom_build_device(const a3d_shape& shape, const GridDev& gd, double h, doubl
   if ((e = temp_alloc(&d_shape, sizeof(a3d_shape), st)) != cudaSuccess) { fail(e, "device memory (shape)"); return rc; }
   if ((e = temp_alloc(&cin, nodes, st)) != cudaSuccess) fail(e, "device memory (node flags)");
   if (rc == A3D_OK && (e = temp_alloc(&mark, N, st)) != cudaSuccess) fail(e, "device memory (marks)");
-  if (rc == A3D_OK && (e = temp_alloc(&d_cnt, 2 * sizeof(unsigned long long), st)) != cudaSuccess) fail(e, "device memory (counts)");
+  if (rc == A3D_OK && (e = temp_alloc(&d_cnt, 3 * sizeof(unsigned long long), st)) != cudaSuccess) fail(e, "device memory (counts)");
   if (rc == A3D_OK) {
     GeoDev g;
     g.a = d_shape;
@@ -286,51 +378,38 @@ int geom_build_device(const a3d_shape& shape, const GridDev& gd, double h, doubl
     if (vol) { vol[0] = g.volW; vol[1] = g.volH; vol[2] = g.volV; }
     cudaMemcpyAsync(d_shape, &shape, sizeof(a3d_shape), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(mark, 0, N, st);
+    cudaMemsetAsync(d_cnt, 0, 3 * sizeof(unsigned long long), st);
     k_nodes<<<grid_blocks(nodes), 256, 0, st>>>(g, cin);
-    k_cells<<<grid_blocks(N), 256, 0, st>>>(g, cin, out.phi, out.ap0, out.ap1, out.ap2, out.ap3);
-    k_baffle<<<grid_blocks((long)NX * NY), 256, 0, st>>>(g, 0, out.ap2, out.ap3);
-    k_baffle<<<grid_blocks((long)NX * NY), 256, 0, st>>>(g, 1, out.ap2, out.ap3);
-    k_solid<<<grid_blocks(N), 256, 0, st>>>(N, out.phi, out.t);
-    // fixed-state layers, in the reference's engine/exit order; a layer that catches no cell
-    // centre is marked again with a padded ring (src/air_cfd.js:124, 129)
+    k_cells<<<grid_blocks(N), 256, 0, st>>>(g, cin, out.phi, out.ap0, out.ap1, out.ap2, out.ap3, out.t);
+    k_baffle<<<grid_blocks(((long)NX * NY + 2) / 3 * 32), 256, 0, st>>>(g, out.ap2, out.ap3);
+    // fixed-state layers, in the reference's engine/exit order
     auto layer_at = [&](double xv) { int i = 0; while (i < NX - 1 && gd.hXf[i + 1] <= xv) i++; return i; };
-    auto mark_ring = [&](int i, const a3d_engine& E, double rin, double rout, int ty, uint8_t bit, unsigned long long& n) {
-      cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), st);
-      k_mark<<<grid_blocks((long)NY * NZ), 256, 0, st>>>(g, i, E.y, E.z, rin, rout, ty, bit, out.t, out.phi, mark, d_cnt);
-      cudaMemcpyAsync(&n, d_cnt, sizeof(n), cudaMemcpyDeviceToHost, st);
-      return cudaStreamSynchronize(st);
-    };
-    for (int en = 0; en < shape.n_engines && rc == A3D_OK; en++) {
+    Rings rings;
+    rings.n = 0;
+    for (int en = 0; en < std::min<int>(shape.n_engines, A3D_MAX_ENGINES); en++) {
       const a3d_engine& E = shape.engines[en];
-      for (int x = 0; x < shape.n_exits && rc == A3D_OK; x++) {
+      const double pad = 0.55 * std::max(std::max((double)gd.hYd0, (double)gd.hZd0), h);
+      for (int x = 0; x < std::min<int>(shape.n_exits, A3D_MAX_EXITS); x++) {
         const a3d_exit& ex = shape.exits[x];
-        const int i = layer_at(E.x0 + ex.x - 1e-3);
-        unsigned long long n = 0;
-        if ((e = mark_ring(i, E, ex.Rin, ex.R, ex.type, 1, n)) != cudaSuccess) { fail(e, "exit layer"); break; }
-        if (!n) {
-          const double pad = 0.55 * std::max(std::max((double)gd.hYd0, (double)gd.hZd0), h);
-          if ((e = mark_ring(i, E, ex.Rin - pad, ex.R + pad, ex.type, 1, n)) != cudaSuccess) fail(e, "exit layer");
-        }
+        rings.r[rings.n++] = {layer_at(E.x0 + ex.x - 1e-3), ex.type, 1,           E.y, E.z, ex.Rin, ex.R,
+                              ex.Rin - pad,                 ex.R + pad};
       }
-      if (!E.internal && rc == A3D_OK) {
-        const int i = layer_at(E.x0 + shape.lip_x + 1e-3);
-        unsigned long long n = 0;
-        // ring test r <= 0.9 lip_r + pad with no inner bound
-        if ((e = mark_ring(i, E, -1e300, 0.9 * shape.lip_r, T_SINK, 2, n)) != cudaSuccess) { fail(e, "intake layer"); break; }
-        if (!n && (e = mark_ring(i, E, -1e300, 0.9 * shape.lip_r + 0.55 * h, T_SINK, 2, n)) != cudaSuccess) fail(e, "intake layer");
+      if (!E.internal) {  // ring test r <= 0.9 lip_r + pad with no inner bound
+        const double r = 0.9 * shape.lip_r;
+        rings.r[rings.n++] = {layer_at(E.x0 + shape.lip_x + 1e-3), T_SINK, 2, E.y, E.z, -1e300, r, -1e300, r + 0.55 * h};
       }
     }
-    if (rc == A3D_OK) {
-      k_cleanup<<<grid_blocks(N), 256, 0, st>>>(NX, NY, NZ, out.t, out.ap0, out.ap1, out.ap2, out.ap3);
-      k_force_open<<<grid_blocks(N), 256, 0, st>>>(N, out.t, mark, out.ap0);
-      cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), st);
-      k_counts<<<grid_blocks(N), 256, 0, st>>>(N, out.t, out.phi, out.ap0, out.ap1, out.ap2, d_cnt);
-      unsigned long long hc[2] = {0, 0};
-      cudaMemcpyAsync(hc, d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, st);
-      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) fail(e, "geometry kernels");
-      else if ((e = cudaGetLastError()) != cudaSuccess) fail(e, "geometry launch");
-      if (counts) { counts[0] = (int64_t)hc[0]; counts[1] = (int64_t)hc[1]; }
+    if (rings.n) {
+      k_ring_caught<<<grid_blocks((long)NY * NZ), 256, 0, st>>>(g, rings, (unsigned*)(d_cnt + 2));
+      k_mark<<<grid_blocks((long)NY * NZ), 256, 0, st>>>(g, rings, (unsigned*)(d_cnt + 2), out.t, out.phi, mark);
     }
+    k_finish<<<(int)std::min<long>(grid_blocks(N), 148 * 8), 256, 0, st>>>(NX, NY, NZ, out.t, out.phi, mark, out.ap0,
+                                                                           out.ap1, out.ap2, out.ap3, d_cnt);
+    unsigned long long hc[2] = {0, 0};
+    if (counts) cudaMemcpyAsync(hc, d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, st);
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) fail(e, "geometry kernels");
+    else if ((e = cudaGetLastError()) != cudaSuccess) fail(e, "geometry launch");
+    if (counts) { counts[0] = (int64_t)hc[0]; counts[1] = (int64_t)hc[1]; }
   }
   cudaFreeAsync(d_cnt, st);
   cudaFreeAsync(mark, st);

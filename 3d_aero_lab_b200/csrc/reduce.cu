@@ -44,41 +44,72 @@ __device__ __forceinline__ bool force_entry(const FlArgs& f, long q, double& cx,
   return cx != 0 || cz != 0;
 }
 
-__global__ void k_fl_count(FlArgs f, long N, int* counts) {
-  const long base = (long)blockIdx.x * kFlPerBlock + (long)threadIdx.x * kFlPerThread;
+// Entries of each block of kFlPerBlock cells; the last block to finish turns them into the blocks'
+// places in the list and writes the list's length to *total (page-locked host memory).
+__global__ void __launch_bounds__(kFlThreads) k_fl_count(FlArgs f, long N, long* offsets, unsigned* finished,
+                                                         double* total) {
+  typedef cub::BlockReduce<int, kFlThreads> BR;
+  typedef cub::BlockScan<long, kFlThreads> BS;
+  __shared__ union { typename BR::TempStorage r; typename BS::TempStorage s; } tmp;
+  __shared__ bool last;
   int n = 0;
   for (int e = 0; e < kFlPerThread; e++) {
+    const long q = (long)blockIdx.x * kFlPerBlock + e * kFlThreads + threadIdx.x;
     double cx, cz;
-    if (base + e < N && force_entry(f, base + e, cx, cz)) n++;
+    if (q < N && force_entry(f, q, cx, cz)) n++;
   }
-  typedef cub::BlockReduce<int, kFlThreads> BR;
-  __shared__ typename BR::TempStorage tmp;
-  const int tot = BR(tmp).Sum(n);
-  if (threadIdx.x == 0) counts[blockIdx.x] = tot;
+  const int tot = BR(tmp.r).Sum(n);
+  if (threadIdx.x == 0) {
+    offsets[blockIdx.x] = tot;
+    __threadfence();
+    last = atomicAdd(finished, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  long before = 0;
+  for (unsigned b0 = 0; b0 < gridDim.x; b0 += kFlThreads) {
+    const unsigned b = b0 + threadIdx.x;
+    const long v = b < gridDim.x ? __ldcg(offsets + b) : 0;
+    long pre, all;
+    BS(tmp.s).ExclusiveSum(v, pre, all);
+    if (b < gridDim.x) offsets[b] = before + pre;
+    before += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    *finished = 0;
+    *total = (double)before;
+  }
 }
 
-__global__ void k_fl_write(FlArgs f, long N, const long* offsets, int64_t* oq, double* ocx, double* ocz,
-                           double* ox, double* oz) {
-  const long base = (long)blockIdx.x * kFlPerBlock + (long)threadIdx.x * kFlPerThread;
-  int n = 0;
-  bool hit[kFlPerThread];
+// The entries in cell order: warp w of a block takes cells [128 w, 128 w + 128), 32 at a time.
+__global__ void __launch_bounds__(kFlThreads) k_fl_write(FlArgs f, long N, const long* offsets, int64_t* oq,
+                                                         double* ocx, double* ocz, double* ox, double* oz) {
+  constexpr int kWarps = kFlThreads / 32;
+  __shared__ int in_warp[kWarps];
+  const int w = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const long base = (long)blockIdx.x * kFlPerBlock + w * (32 * kFlPerThread) + lane;
+  unsigned hits[kFlPerThread];
   double cx[kFlPerThread], cz[kFlPerThread];
+  int n = 0;
   for (int e = 0; e < kFlPerThread; e++) {
-    hit[e] = base + e < N && force_entry(f, base + e, cx[e], cz[e]);
-    n += hit[e];
+    const long q = base + 32 * e;
+    hits[e] = __ballot_sync(0xffffffffu, q < N && force_entry(f, q, cx[e], cz[e]));
+    n += __popc(hits[e]);
   }
-  typedef cub::BlockScan<int, kFlThreads> BS;
-  __shared__ typename BS::TempStorage tmp;
-  int pre;
-  BS(tmp).ExclusiveSum(n, pre);
-  long o = offsets[blockIdx.x] + pre;
+  if (lane == 0) in_warp[w] = n;
+  __syncthreads();
+  long o = offsets[blockIdx.x];
+  for (int v = 0; v < w; v++) o += in_warp[v];
   const long NX = f.NX, NXY = NX * f.NY;
   for (int e = 0; e < kFlPerThread; e++) {
-    if (!hit[e]) continue;
-    const long q = base + e;
-    oq[o] = q; ocx[o] = cx[e]; ocz[o] = cz[e];
-    ox[o] = f.Xc[q % NX]; oz[o] = f.Zc[q / NXY];
-    o++;
+    if (hits[e] >> lane & 1) {
+      const long q = base + 32 * e, p = o + __popc(hits[e] & ((1u << lane) - 1));
+      oq[p] = q; ocx[p] = cx[e]; ocz[p] = cz[e];
+      ox[p] = f.Xc[q % NX]; oz[p] = f.Zc[q / NXY];
+    }
+    o += __popc(hits[e]);
   }
 }
 
@@ -284,40 +315,33 @@ void locate(const std::vector<float>& c, double v, int& i, double& tx) {
 
 }  // namespace
 
+// Queued on the solver's stream; the list's length is known on return.
 int build_force_list(a3d_solver* s) {
   const long N = s->N;
   const long nb = (N + kFlPerBlock - 1) / kFlPerBlock;
   FlArgs f = fl_args(s);
-  int* d_counts = nullptr;
+  const RedArgs red = red_args(s);
   long* d_off = nullptr;
-  A3D_CUDA(dev_alloc(&d_counts, nb * sizeof(int)));
-  std::vector<int> counts(nb);
-  k_fl_count<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_counts);
-  cudaError_t e = cudaMemcpyAsync(counts.data(), d_counts, nb * sizeof(int), cudaMemcpyDeviceToHost, s->st);
+  A3D_CUDA(temp_alloc(&d_off, nb * sizeof(long), s->st));
+  k_fl_count<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_off, red.finished, red.out);
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
-  if (e != cudaSuccess) { dev_free(d_counts); set_error("force list count: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
-  std::vector<long> off(nb);
-  long tot = 0;
-  for (long b = 0; b < nb; b++) { off[b] = tot; tot += counts[b]; }
+  if (e != cudaSuccess) { cudaFreeAsync(d_off, s->st); set_error("force list count: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
+  const long tot = (long)s->h_red[0];
   s->fl.n = tot;
   const size_t n1 = (size_t)std::max(tot, 1L);
   char* blk = nullptr;
   e = dev_alloc(&blk, n1 * (8 + 4 * 8) + 256);
-  if (e == cudaSuccess) e = dev_alloc(&d_off, nb * sizeof(long));
-  if (e != cudaSuccess) { dev_free(d_counts); dev_free(blk); set_error("force list alloc: %s", cudaGetErrorString(e)); return A3D_ERR_NOMEM; }
+  if (e != cudaSuccess) { cudaFreeAsync(d_off, s->st); set_error("force list alloc: %s", cudaGetErrorString(e)); return A3D_ERR_NOMEM; }
   s->fl.block = blk;
   s->fl.q = (int64_t*)blk;
   s->fl.cx = (double*)(blk + n1 * 8);
   s->fl.cz = s->fl.cx + n1;
   s->fl.x = s->fl.cz + n1;
   s->fl.z = s->fl.x + n1;
-  e = cudaMemcpyAsync(d_off, off.data(), nb * sizeof(long), cudaMemcpyHostToDevice, s->st);
-  if (e == cudaSuccess) {
-    k_fl_write<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_off, s->fl.q, s->fl.cx, s->fl.cz, s->fl.x, s->fl.z);
-    e = cudaStreamSynchronize(s->st);
-  }
-  dev_free(d_counts);
-  dev_free(d_off);
+  k_fl_write<<<(unsigned)nb, kFlThreads, 0, s->st>>>(f, N, d_off, s->fl.q, s->fl.cx, s->fl.cz, s->fl.x, s->fl.z);
+  e = cudaGetLastError();
+  cudaFreeAsync(d_off, s->st);
   if (e != cudaSuccess) { set_error("force list write: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
   return A3D_OK;
 }
@@ -428,7 +452,9 @@ extern "C" int a3d_solver_set_owned(a3d_solver* s, int32_t k0, int32_t k1) {
   A3D_CUDA(cudaDeviceSynchronize());  // nothing still reads the list
   dev_free(s->fl.block);
   s->fl = ForceList();
-  return build_force_list(s);
+  A3D_TRY(build_force_list(s));
+  A3D_CUDA(cudaStreamSynchronize(s->st));
+  return A3D_OK;
 }
 
 extern "C" int a3d_solver_residual_parts(a3d_solver* s, double out[2]) {

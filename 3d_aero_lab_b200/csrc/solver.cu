@@ -30,25 +30,29 @@ namespace {
 // ----------------------------------------------------------------------------------------
 // per-cell codes: type, static slope-test bits, irregular and baffle flags
 // ----------------------------------------------------------------------------------------
-__global__ void k_codes(int NX, int NY, int NZ, int NXp, const uint8_t* t, const float* phi, const float* ap0,
-                        const float* ap1, const float* ap2, const float* ap3, uint8_t* code) {
-  const long NXY = (long)NX * NY, N = NXY * NZ;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(q % NX), j = (int)((q / NX) % NY), k = (int)(q / NXY);
-    uint8_t c = t[q] & 7;
-    auto fluid = [&](long qq) { return t[qq] == T_FLUID; };
+__global__ void k_codes(int NX, int NY, int NZ, int NXp, const uint8_t* __restrict__ t, const float* __restrict__ phi,
+                        const float* __restrict__ ap0, const float* __restrict__ ap1, const float* __restrict__ ap2,
+                        const float* __restrict__ ap3, uint8_t* __restrict__ code) {
+  // (a solver's grid has fewer than 2^31 cells)
+  const uint32_t NXY = (uint32_t)NX * NY, N = NXY * NZ;
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
+    const uint32_t row = q / (uint32_t)NX;
+    const int i = (int)(q - row * NX), k = (int)(row / (uint32_t)NY), j = (int)(row - (uint32_t)k * NY);
+    const uint8_t tq = t[q];
+    const bool in = tq == T_FLUID;
+    // the six faces and their cells; a domain edge's face is open, its ghost never fluid
+    const float xp = ap0[q], yp = ap1[q], zp = ap2[q], b = ap3[q];
+    const float xm = i > 0 ? ap0[q - 1] : 1.f, ym = j > 0 ? ap1[q - NX] : 1.f, zm = k > 0 ? ap2[q - NXY] : 1.f;
+    const float bm = k > 0 ? ap3[q - NXY] : 0.f;
+    uint8_t c = tq & 7;
     // slope allowed at this cell along d: both neighbours in the domain and fluid, this cell
     // fluid, both faces fully open (src/air_cfd.js:214; out-of-domain ghosts are never fluid)
-    if (t[q] == T_FLUID) {
-      if (i > 0 && i + 1 < NX && fluid(q - 1) && fluid(q + 1) && ap0[q - 1] == 1.f && ap0[q] == 1.f) c |= C_OKX;
-      if (j > 0 && j + 1 < NY && fluid(q - NX) && fluid(q + NX) && ap1[q - NX] == 1.f && ap1[q] == 1.f) c |= C_OKY;
-      if (k > 0 && k + 1 < NZ && fluid(q - NXY) && fluid(q + NXY) && ap2[q - NXY] == 1.f && ap2[q] == 1.f) c |= C_OKZ;
-    }
-    if (phi[q] != 1.f || ap0[q] != 1.f || ap1[q] != 1.f || ap2[q] != 1.f || (i > 0 && ap0[q - 1] != 1.f) ||
-        (j > 0 && ap1[q - NX] != 1.f) || (k > 0 && ap2[q - NXY] != 1.f))
-      c |= C_IRR;
-    if (ap3[q] != 0.f || (k > 0 && ap3[q - NXY] != 0.f)) c |= C_BAF;
-    code[((long)k * NY + j) * NXp + i] = c;
+    if (in && i > 0 && i + 1 < NX && xm == 1.f && xp == 1.f && t[q - 1] == T_FLUID && t[q + 1] == T_FLUID) c |= C_OKX;
+    if (in && j > 0 && j + 1 < NY && ym == 1.f && yp == 1.f && t[q - NX] == T_FLUID && t[q + NX] == T_FLUID) c |= C_OKY;
+    if (in && k > 0 && k + 1 < NZ && zm == 1.f && zp == 1.f && t[q - NXY] == T_FLUID && t[q + NXY] == T_FLUID) c |= C_OKZ;
+    if (phi[q] != 1.f || xp != 1.f || yp != 1.f || zp != 1.f || xm != 1.f || ym != 1.f || zm != 1.f) c |= C_IRR;
+    if (b != 0.f || bm != 0.f) c |= C_BAF;
+    code[(size_t)row * NXp + i] = c;
   }
 }
 

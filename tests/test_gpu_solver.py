@@ -325,6 +325,28 @@ def test_postprocessing_matches_oracle(aero, ref):
     assert math.isclose(s.residual(3), o.residual(3), rel_tol=1e-9)
 
 
+@pytest.mark.parametrize("cells", [700, 8000, 400000, 1500000])
+def test_force_list_is_every_entry_in_cell_order(aero, cells):
+    """From one block of cells to more blocks than one turn of the scan takes: the entries that the
+    geometry arrays give (src/air_cfd.js:143-152), in cell order and to the last bit."""
+    sh = aero.shape_of(aero.build_aircraft("airliner"))
+    g, s = gpu_case(aero, sh, cells, 2.0)
+    ge = aero.cfd_geom(sh, g, 2.0)
+    shp = (g.NZ, g.NY, g.NX)
+    a0, a2 = (ge.ap[d].reshape(shp).astype(np.float64) for d in (0, 2))
+    xd, yd, zd = (np.diff(f).astype(np.float32).astype(np.float64) for f in (g.X.f, g.Y.f, g.Z.f))
+    dx, dz = a0.copy(), a2.copy()
+    dx[:, :, 1:] -= a0[:, :, :-1]
+    dx[:, :, 0] -= 1
+    dz[1:] -= a2[:-1]
+    dz[0] -= 1
+    cx = (dx * yd[None, :, None] * zd[:, None, None]).ravel()
+    cz = (dz * xd[None, None, :] * yd[None, :, None]).ravel()
+    q = np.nonzero((ge.t.ravel() == 0) & ((cx != 0) | (cz != 0)))[0]
+    fl = s.force_list()
+    assert np.array_equal(fl["q"], q) and np.array_equal(fl["cx"], cx[q]) and np.array_equal(fl["cz"], cz[q])
+
+
 @pytest.mark.parametrize("cells", [8000, 70000, 1500000])
 def test_residual_strides_and_snapshots(aero, cells):
     """One pass samples every stride-th fluid cell and takes the next call's snapshot, from less than
