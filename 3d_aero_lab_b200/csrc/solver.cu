@@ -258,16 +258,18 @@ int launch_stage(a3d_solver* s, const StageArgs& a, bool dependent) {
 
 namespace {
 
-// Number of pipelined z chunks a3d_solver_step uses: kernels 2 and 4 on a whole case only.  Automatic:
-// four chunks from 0.8M cells up, where a stage takes long enough to hide the extra stream and
-// event calls (measured: 4.1M-cell fighter 13.5 -> 15.1 G cell-updates/s, 1.0M-cell airliner
-// 10.1 -> 11.2), none below (0.6M-cell interceptor 8.4 -> 8.1 with four).
+// Number of pipelined z chunks a3d_solver_step uses: kernels 2 and 4 on a whole case only.
 int chunk_count(const a3d_solver* s) {
   if ((s->kernel != KERNEL_TMA && s->kernel != KERNEL_PAIR) || s->nbr[0] || s->nbr[1] || s->own_k0 != 0 ||
       s->own_k1 != s->grid.NZ)
     return 1;
   const int runs = (s->grid.NZ + s->march_kz - 1) / s->march_kz;
-  const int K = s->chunks_req > 0 ? s->chunks_req : (s->N >= 800000 ? 4 : 1);
+  // One launch per stage, each dependent on the one before, holds up to 0.95M cells (us per iteration,
+  // its run's launch / three chunks of 3 planes: 675k 53.5 / 57.3, 745k 59.0 / 60.0, 825k 61.2 / 61.1 and
+  // 58.7 / 60.1, 914k 69.6 / 69.5 and 61.5 / 63.4, 933k 69.7 / 67.4, 1.1M 84.6 / 82.5 and 79.8 / 73.7).
+  // Three chunks beat four while a chunk is less than a wave of 10-plane runs (us per iteration, 3 / 4:
+  // 1.1M 82 / 88, 1.8M 126 / 132, 2.4M 150 / 157; 3.0M 180 / 178, 4.0M 228 / 228, 9.1M 442 / 438)
+  const int K = s->chunks_req > 0 ? s->chunks_req : s->N >= 2700000 ? 4 : s->N >= kChunkCells ? 3 : 1;
   return std::max(1, std::min(K, std::min(runs, (int)kMaxChunks)));
 }
 
@@ -544,7 +546,7 @@ int step_chunked(a3d_solver* s, int n, int K) {
 
 }  // namespace
 
-// Pipelined z chunks of a3d_solver_step (kernel 2): 0 = automatic (4 from 0.8M cells up, else 1),
+// Pipelined z chunks of a3d_solver_step (kernel 2): 0 = automatic (4 from 2.7M cells up, 3 from 0.95M, else 1),
 // 1 = one launch per stage, 2..4 = that many chunks.  Results do not depend on it.
 extern "C" int a3d_solver_set_chunks(a3d_solver* s, int32_t chunks) {
   clear_error();
@@ -783,18 +785,54 @@ extern "C" int a3d_solver_write(a3d_solver* s, const float* r, const float* ru, 
   return A3D_OK;
 }
 
+namespace {
+
+// z planes per CTA of the single-cell tile: 32 where that still launches four waves of CTAs (column
+// tiles x z runs >= 4 x resident CTAs), else the longest run of 16, 8 or 4 planes that launches two
+// waves, else 2.
+int auto_run_tma(long columns, int NZ, int resident) {
+  auto ctas = [&](int kz) { return columns * ((NZ + kz - 1) / kz); };
+  if (ctas(32) >= 4L * resident) return 32;
+  for (int kz : {16, 8, 4})
+    if (ctas(kz) >= 2L * resident) return kz;
+  return 2;
+}
+
+// z planes per CTA of the paired tile.  A run costs its planes and half a plane of prologue beyond
+// them; a stage costs its waves of CTAs.
+// Pipelined z chunks (0.95M cells up): the next stage fills the tail, so what counts is runs long
+// enough to carry their prologue and short enough for the chunks to overlap: 2.5 waves, 3 to 32
+// planes.  us per iteration at 2.5 waves against the longest power of two with 2 waves: 1.1M 82 / 88
+// (4 planes, 4 in four chunks), 1.8M 126 / 132 (5, 4), 2.4M 150 / 157 (6, 8), 3.0M 178 / 187 (12, 8),
+// 4.0M 227 / 236 (12, 8), 16M 778 / 793 (32, 16).
+// One launch per stage: the run with the least time by waves, where a last wave of n of the chip's
+// CTAs costs a share 0.55 + 0.9 n of a full one (fewer CTAs on an SM run faster), and one of the last,
+// short runs only costs what does not fit in the half run's time by which the edge tiles are done.
+// Over 48 grids of 22k to 0.95M cells of three types the run picked is 0.9 % slower than the fastest
+// of 1..12 on average, 11 % at most; 2 planes wherever single ones are more than a wave: 4.0 %, 21 %.
+// us per iteration, picked / 2 planes: 268k 32.0 / 38.6 (3 planes), 522k 46.2 / 52.2 (5), 675k 53.5 /
+// 59.8 (6); single planes up to one wave: 31k 17.9 against 24.6.
+int auto_run_pair(long columns, int NZ, long cells, int resident) {
+  if (cells >= kChunkCells) return (int)std::clamp(std::lround(columns * NZ / (2.5 * resident)), 2L, 32L);
+  int best = 1;
+  double least = INFINITY;
+  for (int kz = 1; kz <= std::min(NZ, 16); kz++) {
+    const int runs = (NZ + kz - 1) / kz, shortest = NZ - (runs - 1) * kz;
+    const long full = columns * runs / resident, rest = columns * runs % resident;
+    const double run = kz + 0.5;
+    double t = full * run;
+    if (full == 0) t = run;
+    else if (rest > columns) t += std::min(1.0, 0.55 + 0.9 * rest / resident) * run;
+    else if (rest > 0) t += std::max(0.0, shortest + 0.5 - 0.5 * run);
+    if (t < least) { least = t; best = kz; }
+  }
+  return best;
+}
+
+}  // namespace
+
 // Selects the stage kernel (0: per-cell, 2: TMA tile, 4: paired-cell TMA tile) and the z planes
-// per CTA of the tiled kernels.  march_kz = 0 picks it for the TMA tiles: 32 planes where that still
-// launches four waves of CTAs (column tiles x z runs >= 4 x resident CTAs), else the longest run
-// of 16, 8 or 4 planes that launches two waves, else 2.  Shorter runs cost more ring prologue
-// per plane but keep the SMs busy and the z chunks of a3d_solver_step overlapping.  Measured
-// (G cell-updates/s, fighter): 15.8M cells 32 planes 16.0 (16: 15.7); 4.1M 16 planes 15.1 (32:
-// 13.8); 2.0M 8 planes 13.5 (16: 12.2); 1.0M 4 planes 12.6 (8: 11.8); 0.3M 2 planes 7.3 (8:
-// 5.6); 31k 2 planes 1.5 (8: 0.7).
-// The paired tile takes single planes where all of them fit the chip at once: the stage is then
-// one CTA's latency, and a plane less in it counts for more than the planes read twice (us per
-// iteration, 1 plane against 2: 20k cells 16.4 / 24.1, 31k 17.9 / 24.6, 98k, 258 of 296 resident
-// CTAs, 20.5 / 24.6; beyond one wave it turns, 150k, 396 CTAs, 32.8 / 28.7).
+// per CTA of the tiled kernels (march_kz = 0: by the rules above).
 // Not part of the reference surface.
 extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t march_kz) {
   clear_error();
@@ -811,13 +849,8 @@ extern "C" int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t marc
       A3D_CUDA(cudaSetDevice(s->device));
       if (kernel == KERNEL_PAIR) A3D_TRY(pair_resident_ctas(&resident));
       else A3D_TRY(tma_resident_ctas(&resident));
-      auto ctas = [&](int kz) { return columns * ((s->grid.NZ + kz - 1) / kz); };
-      march_kz = 2;
-      if (ctas(32) >= 4L * resident) march_kz = 32;
-      else if (kernel == KERNEL_PAIR && ctas(1) <= resident) march_kz = 1;
-      else
-        for (int kz : {16, 8, 4})
-          if (ctas(kz) >= 2L * resident) { march_kz = kz; break; }
+      march_kz = kernel == KERNEL_PAIR ? auto_run_pair(columns, s->grid.NZ, s->N, resident)
+                                       : auto_run_tma(columns, s->grid.NZ, resident);
     }
   }
   s->kernel = kernel;

@@ -48,6 +48,7 @@ struct ForceList {
 // Stage kernels by number (the numbers 1 and 3 belonged to two tiles since retired: slower
 // than the TMA tiles on every measured case).
 enum StageKernel { KERNEL_CELL = 0, KERNEL_TMA = 2, KERNEL_PAIR = 4 };
+constexpr long kChunkCells = 950000;  // from here on a step runs as z chunks
 constexpr int kMaxChunks = 4;  // z chunks of a pipelined step (6 or 8 measured no faster)
 
 }  // namespace a3d

@@ -185,9 +185,10 @@ int a3d_solver_interp_state(a3d_solver* fine, const a3d_solver* coarse);
  * kernel 4 (default): the same over 32 x 16-column tiles, each thread two x-adjacent cells
  *           in packed f32x2 arithmetic, two CTAs per SM.
  * (Numbers 1 and 3 belonged to two tiles since retired; they are refused.)
- * march_kz = z planes per thread block; 0 (the default) picks for the TMA tiles 32 planes if
- * that still launches four waves of CTAs, else (kernel 4) single planes if all their CTAs are
- * resident at once, else the longest of 16, 8 or 4 planes that launches two waves, else 2. */
+ * march_kz = z planes per thread block; 0 (the default) picks it from the grid and the chip:
+ * for kernel 4 the run (at most 16 planes) whose waves of thread blocks take the least time, or,
+ * where a step runs as z chunks, 2.5 waves of runs of 3 to 32 planes; for kernel 2 32 planes if
+ * that still launches four waves, else the longest of 16, 8 or 4 that launches two, else 2. */
 int a3d_solver_set_kernel(a3d_solver* s, int32_t kernel, int32_t march_kz);
 int a3d_solver_get_kernel(a3d_solver* s, int32_t* kernel, int32_t* march_kz);
 /* Bounded device waits; no counterpart in the reference.  Every wait of a stage kernel (the
@@ -200,7 +201,7 @@ int a3d_solver_get_kernel(a3d_solver* s, int32_t* kernel, int32_t* march_kz);
 int a3d_solver_set_wait_limit(a3d_solver* s, uint32_t limit);
 /* Kernels 2 and 4 step the case as up to 4 z chunks of whole z runs on their own streams, each
  * chunk's stage waiting only for its neighbour chunks' previous stage: the tail of one stage
- * overlaps the start of the next.  0 = automatic (4 chunks from 0.8M cells up, else 1),
+ * overlaps the start of the next.  0 = automatic (4 chunks from 2.7M cells up, 3 from 0.95M, else 1),
  * 1 = one launch per stage, 2..4 = that many chunks.  The results are the same bit for bit. */
 int a3d_solver_set_chunks(a3d_solver* s, int32_t chunks);
 /* The number of chunks (stage launches per RK stage) a3d_solver_step uses for this case.  */

@@ -150,6 +150,22 @@ def test_automatic_z_run_takes_single_planes_on_one_wave(aero, cells, kz):
     assert max(rel_max_diff(A[c], B[c]) for c in range(5)) < 4e-6
 
 
+@pytest.mark.parametrize("cells", [30000, 181000, 270000, 522000, 820000, 1000000, 2000000, 2900000])
+def test_automatic_runs_and_chunks_leave_the_bits(aero, cells):
+    """The automatic z run and number of z chunks, over each branch of their rules, against 11-plane
+    runs in one launch per stage: which CTA computes a plane changes nothing."""
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    g, a = gpu_case(aero, sh, cells, 1.0)
+    _, b = gpu_case(aero, sh, cells, 1.0)
+    assert 1 <= a.kernel()[1] <= min(32, g.NZ)
+    assert a.chunks() == (1 if g.N < 950000 else 3 if g.N < 2700000 else 4)
+    b.set_kernel(4, 11)
+    b.set_chunks(1)
+    a.step(6)
+    b.step(6)
+    assert np.array_equal(a.read_array(), b.read_array())
+
+
 @pytest.mark.parametrize("kernel", [2, 4])
 def test_bounded_wait_runs_out_reports_timeout_and_recovers(aero, kernel):
     """The TMA tiles' bounded waits (SURVEY failure detection): with the wait limit at 0 every wait
