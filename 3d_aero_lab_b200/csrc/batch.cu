@@ -86,8 +86,9 @@ __device__ __forceinline__ void batch_loop(unsigned char* smem_raw, const BatchC
     const bool ok = TILE == TILE_TMA
                         ? tma::stage_tile<STAGE2, true>(*reinterpret_cast<tma::TmaSmem*>(smem_raw), &C.tmQ[qin], &C.tmC,
                                                         s_a, C.buf[iq], out, bx, by, bz, C.kz)
-                        : pair::stage_tile<STAGE2, true>(*reinterpret_cast<pair::PairSmem*>(smem_raw), &C.tmQ[qin],
-                                                         &C.tmC, s_a, C.buf[iq], out, bx, by, bz, C.kz);
+                        : pair::stage_tile<STAGE2, true>(*reinterpret_cast<pair::PairSmem*>(smem_raw),
+                                                         pair::Maps{&C.tmQ[qin], &C.tmC, nullptr, nullptr}, s_a,
+                                                         C.buf[iq], out, bx, by, bz, C.kz);
     if (!ok) {
       if (threadIdx.x == 0) {
         s_failed = 1;

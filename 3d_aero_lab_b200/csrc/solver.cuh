@@ -75,6 +75,7 @@ struct a3d_solver {
   CUtensorMap tmC;                // TMA map over the code array
   CUtensorMap tmQp[3];            // the same maps with the paired tile's boxes (32 x 16 columns + halo)
   CUtensorMap tmCp;
+  CUtensorMap tmQo[3], tmCo;      // and its bare columns, without the halo
   uint32_t wait_limit = A3D_WAIT_LIMIT_DEFAULT;  // try_waits a stage kernel spends on one TMA copy
   int march_kz = 16;              // z planes per CTA of the marching kernels
   bool kz_auto = true;            // picked from the grid size, not by the caller

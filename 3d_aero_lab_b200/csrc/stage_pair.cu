@@ -10,16 +10,18 @@ namespace {
 
 using namespace pair;
 
-// At most 128 registers: two CTAs (16 warps) per SM.  MODE 0: all planes of the case; 1: planes
-// [a.kb, a.ke) (a z chunk or a slab's own planes); 2: the same with the halo push of a z slab.
+// At most 128 registers: two CTAs (16 warps) per SM.  MODE 0: all planes of a lone case, dependent on
+// the launch before; 1: planes [a.kb, a.ke) (a z chunk, a slab's own planes, a case of a batch); 2: the
+// same with the halo push of a z slab.
 template <bool STAGE2, int MODE>
 __global__ void __launch_bounds__(NT, 2)
-    k_stage_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC, StageArgs a,
+    k_stage_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC,
+                 const __grid_constant__ CUtensorMap tmQo, const __grid_constant__ CUtensorMap tmCo, StageArgs a,
                  int kz) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   PairSmem& S = *reinterpret_cast<PairSmem*>(smem_raw);
-  stage_tile<STAGE2, false, MODE >= 1, MODE == 2>(S, &tmQ, &tmC, a, a.B, a.Out, blockIdx.x, blockIdx.y, blockIdx.z,
-                                                  kz);
+  stage_tile<STAGE2, false, MODE >= 1, MODE == 2>(S, Maps{&tmQ, &tmC, &tmQo, &tmCo}, a, a.B, a.Out, blockIdx.x,
+                                                  blockIdx.y, blockIdx.z, kz);
 }
 
 template <bool STAGE2, int MODE>
@@ -43,8 +45,10 @@ void launch_mode(const a3d_solver* s, const StageArgs& a, int qin_buf, bool stag
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = dependent ? 1 : 0;
-  if (stage2) cudaLaunchKernelEx(&cfg, k_stage_pair<true, MODE>, s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
-  else cudaLaunchKernelEx(&cfg, k_stage_pair<false, MODE>, s->tmQp[qin_buf], s->tmCp, a, s->march_kz);
+  if (stage2) cudaLaunchKernelEx(&cfg, k_stage_pair<true, MODE>, s->tmQp[qin_buf], s->tmCp, s->tmQo[qin_buf], s->tmCo, a,
+                                   s->march_kz);
+  else cudaLaunchKernelEx(&cfg, k_stage_pair<false, MODE>, s->tmQp[qin_buf], s->tmCp, s->tmQo[qin_buf], s->tmCo, a,
+                                   s->march_kz);
 }
 
 }  // namespace
@@ -65,8 +69,8 @@ int pair_resident_ctas(int* n) {
   return A3D_OK;
 }
 
-// Tensor maps of the paired tile: boxes 40 x 20 x 1 x 5 over the padded state buffers and
-// 64 x 20 x 1 over the code array.
+// Tensor maps of the paired tile: boxes 40 x 20 x 1 x 5 over the padded state buffers and 64 x 20 x 1
+// over the code array, and the bare columns' 32 x 16 x 1 x 5 and 32 x 16 x 1.
 int make_pair_tensor_maps(a3d_solver* s) {
   auto enc = tensor_map_encoder();
   if (!enc) { set_error("cuTensorMapEncodeTiled is not available from the driver"); return A3D_ERR_CUDA; }
@@ -78,12 +82,21 @@ int make_pair_tensor_maps(a3d_solver* s) {
     CUresult r = enc(&s->tmQp[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, s->buf[b], dims, strides, box, es,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t bare[4] = {TX, TY, 1, 5};
+    if (r == CUDA_SUCCESS)
+      r = enc(&s->tmQo[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, s->buf[b], dims, strides, bare, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(pair state) failed: %d", (int)r); return A3D_ERR_CUDA; }
   }
   const cuuint64_t cd[3] = {NX, NY, NZ}, cs[2] = {NXp, NXp * NY};
   const cuuint32_t cb[3] = {CBX, HY, 1}, ce[3] = {1, 1, 1};
   CUresult r = enc(&s->tmCp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, s->code, cd, cs, cb, ce, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint32_t bare[3] = {TX, TY, 1};
+  if (r == CUDA_SUCCESS)
+    r = enc(&s->tmCo, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, s->code, cd, cs, bare, ce, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(pair codes) failed: %d", (int)r); return A3D_ERR_CUDA; }
   A3D_TRY((set_attributes<false, 0>()));
   A3D_TRY((set_attributes<true, 0>()));
@@ -100,9 +113,9 @@ int launch_pair(a3d_solver* s, const StageArgs& a, int qin_buf, bool stage2, cud
   const int kz = s->march_kz;
   dim3 grid((a.NX + TX - 1) / TX, (a.NY + TY - 1) / TY, (a.ke - a.kb + kz - 1) / kz);
   if (!st) st = s->st;
-  if (a.peer[0] || a.peer[1]) launch_mode<2>(s, a, qin_buf, stage2, grid, st, dependent);
-  else if (a.kb != 0 || a.ke != a.NZ) launch_mode<1>(s, a, qin_buf, stage2, grid, st, dependent);
-  else launch_mode<0>(s, a, qin_buf, stage2, grid, st, dependent);
+  if (a.peer[0] || a.peer[1]) launch_mode<2>(s, a, qin_buf, stage2, grid, st, false);
+  else if (dependent && a.kb == 0 && a.ke == a.NZ) launch_mode<0>(s, a, qin_buf, stage2, grid, st, true);
+  else launch_mode<1>(s, a, qin_buf, stage2, grid, st, false);
   A3D_CUDA(cudaGetLastError());
   return A3D_OK;
 }

@@ -19,7 +19,8 @@
 //
 // The planes arrive through a 4-deep ring of shared-memory slots filled by
 // `cp.async.bulk.tensor` (one 40 x 20 x 5-component state box and one 64 x 20 code box per
-// plane, completing on the slot's mbarrier; no cluster multicast).  Per plane k:
+// plane, completing on the slot's mbarrier; no cluster multicast; planes beyond a single launch's
+// runs without the halo).  Per plane k:
 //   [A] plane-k primitives to shared memory (own pair from the column registers, the 2-cell
 //       halo - no corners, which no face reads - by warps 0-2 from the slot); barrier;
 //       thread 0 queues plane k+3 into the slot plane k-1 has left;
@@ -76,18 +77,36 @@ struct PairSmem {
 __device__ __forceinline__ int slot_of(int p, int k0) { return (p - k0 + 2) & (NSLOT - 1); }
 __device__ __forceinline__ uint32_t parity_of(int p, int k0) { return ((p - k0 + 2) / NSLOT) & 1; }
 
+// Tensor maps of a tile: the boxes with the halo, and (Qo, Co; null: none) the bare 32 x 16 columns.
+struct Maps {
+  const CUtensorMap *Q, *C, *Qo, *Co;
+};
+// Planes outside the run only take part in the z slopes of the tile's own columns, so they can come
+// without the halo: 80 rows of one 128-byte line instead of 100 of three, packed from the slot's start.
+// Short runs are mostly such planes (four of five at one plane) and wait for them first.  us per
+// iteration before / with it: 31k 17.9 / 16.8, 100k 17.9 / 17.1, 150k 26.4 / 25.1, 0.55M 56.8 / 56.2,
+// 0.82M 61.1 / 60.3.  In z chunks, whose runs are longer, the choice costs more than it saves (4.1M 227
+// / 229), and so in the batches' 16-plane runs (20.7 / 20.9 ms): they keep the halo on every plane.
+constexpr uint32_t kQoBytes = 5 * TY * TX * 4, kCoBytes = TY * TX;
+
 // Thread 0 queues plane p into its slot: one state box and one code box, or a bare arrive
 // when the plane lies outside the domain (its cells are then all far-field ghosts).
-__device__ __forceinline__ void issue_plane(PairSmem& S, const CUtensorMap* tmQ, const CUtensorMap* tmC,
-                                            const StageArgs& a, int p, int k0, int i0, int j0) {
+__device__ __forceinline__ void issue_plane(PairSmem& S, const Maps& m, const StageArgs& a, int p, int k0, bool outer,
+                                            int i0, int j0) {
   const int s = slot_of(p, k0);
   if (p < 0 || p >= a.NZ) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&S.bar[s])) : "memory");
     return;
   }
+  if (outer) {
+    mbar_expect_tx(&S.bar[s], kQoBytes + kCoBytes);
+    tma_load_4d(&S.slot[s].Q[0][0][0], m.Qo, &S.bar[s], i0, j0, p, 0);
+    tma_load_3d(&S.slot[s].C[0][0], m.Co, &S.bar[s], i0, j0, p);
+    return;
+  }
   mbar_expect_tx(&S.bar[s], kQBytes + kCBytes);
-  tma_load_4d(&S.slot[s].Q[0][0][0], tmQ, &S.bar[s], i0 - 4, j0 - 2, p, 0);
-  tma_load_3d(&S.slot[s].C[0][0], tmC, &S.bar[s], i0 - 16, j0 - 2, p);
+  tma_load_4d(&S.slot[s].Q[0][0][0], m.Q, &S.bar[s], i0 - 4, j0 - 2, p, 0);
+  tma_load_3d(&S.slot[s].C[0][0], m.C, &S.bar[s], i0 - 16, j0 - 2, p);
 }
 
 // A wait ran out: flag the error for the host and wait (bounded, full limit) for the copies
@@ -98,22 +117,16 @@ __device__ __forceinline__ void drain(PairSmem& S, const StageArgs& a, int k0, i
   for (int p = first_pending; p <= last_issued; p++) mbar_wait(&S.bar[slot_of(p, k0)], parity_of(p, k0));
 }
 
-// Primitive states and codes of cells (x, x+1) of row j in the resident plane k (slot s), x
-// even, with the ghost rules of src/air_cfd.js:205-210: far field outside x, z and +y, the
-// symmetry mirror with v negated below y = 0, the fixed state in fixed-state cells (type >= 3).
-// INSIDE: the caller knows both cells lie inside the domain (no ghost tests).  Codes: first
-// cell in the low byte; ghosts T_GHOST, mirror cells T_MIRROR (no slope or aperture bits).
+// Primitive states P and codes of cells (x, x+1) of row j, plane k, from their conservative states q
+// and codes c as the slot holds them, x even, with the ghost rules of src/air_cfd.js:205-210: far
+// field beyond the domain in x, z and +y, the symmetry mirror with v negated below y = 0, the fixed
+// state in fixed-state cells (type >= 3).  INSIDE: the caller knows both cells lie inside the domain
+// (no ghost tests).  Codes: first cell in the low byte; ghosts T_GHOST, mirror cells T_MIRROR (no
+// slope or aperture bits).
 template <bool INSIDE>
-__device__ __forceinline__ uint32_t slot_pair(const StageArgs& a, const Slot& s, int x, int j, int k, int i0, int j0,
-                                              f2 P[5]) {
+__device__ __forceinline__ uint32_t convert(const StageArgs& a, const f2 q[5], uint32_t c, int x, int j, int k,
+                                            f2 P[5]) {
   const bool mirror = !INSIDE && j < 0;
-  // for every pair a tile reads these slot positions stay inside the slot; whatever a ghost's
-  // position holds (another plane, or nothing loaded) is replaced below
-  const int ys = (mirror ? -1 - j : j) - j0 + 2, xs = x - i0 + 4;
-  const uint32_t c = *reinterpret_cast<const uint16_t*>(&s.C[ys][x - i0 + 16]);
-  f2 q[5];
-#pragma unroll
-  for (int v = 0; v < 5; v++) q[v] = *reinterpret_cast<const float2*>(&s.Q[v][ys][xs]);
   prim2(q, P);
   const uint32_t t0 = c & 7, t1 = (c >> 8) & 7;
   if (INSIDE) {
@@ -145,6 +158,28 @@ __device__ __forceinline__ uint32_t slot_pair(const StageArgs& a, const Slot& s,
   const uint32_t e0 = g0 ? (uint32_t)T_GHOST : mirror ? (uint32_t)T_MIRROR : (c & 0xFF);
   const uint32_t e1 = g1 ? (uint32_t)T_GHOST : mirror ? (uint32_t)T_MIRROR : (c >> 8);
   return e0 | (e1 << 8);
+}
+
+// The same from the resident plane k (slot s).  outer: the slot holds the bare columns.
+template <bool INSIDE>
+__device__ __forceinline__ uint32_t slot_pair(const StageArgs& a, const Slot& s, int x, int j, int k, bool outer,
+                                              int i0, int j0, f2 P[5]) {
+  f2 q[5];
+  uint32_t c;
+  if (outer) {
+    const int o = (j - j0) * TX + (x - i0);
+    c = *reinterpret_cast<const uint16_t*>(&s.C[0][0] + o);
+#pragma unroll
+    for (int v = 0; v < 5; v++) q[v] = *reinterpret_cast<const float2*>(&s.Q[0][0][0] + o + v * (TX * TY));
+  } else {
+    // for every pair a tile reads these slot positions stay inside the slot; whatever a ghost's
+    // position holds (another plane, or nothing loaded) is replaced by convert
+    const int ys = (!INSIDE && j < 0 ? -1 - j : j) - j0 + 2, xs = x - i0 + 4;
+    c = *reinterpret_cast<const uint16_t*>(&s.C[ys][x - i0 + 16]);
+#pragma unroll
+    for (int v = 0; v < 5; v++) q[v] = *reinterpret_cast<const float2*>(&s.Q[v][ys][xs]);
+  }
+  return convert<INSIDE>(a, q, c, x, j, k, P);
 }
 
 // Fluxes of two cells' +faces times their apertures, where the codes say that one may differ from 1.
@@ -320,16 +355,16 @@ __device__ __forceinline__ void store_pair(const StageArgs& a, float* __restrict
 }
 
 // One tile: columns (bx, by), planes [bz*kz, bz*kz + kz).  Stage 1 reads the state through
-// tmQ; stage 2 also reads the base state Bp; the result goes to Outp.  Returns false if a
+// the maps; stage 2 also reads the base state Bp; the result goes to Outp.  Returns false if a
 // bounded wait ran out (flagged in *a.err); the CTA's copies in flight are then drained.
 // PERSISTENT: the CTA runs further tiles after this one, so the tile starts with a barrier and
 // retires its ring barriers at the end.  RANGE: the z runs cover planes [a.kb, a.ke) only (a z
-// slab's own planes, or one z chunk of a pipelined step).  PUSH: stores also go to the
+// slab's own planes, one z chunk of a pipelined step, a case of a batch), ordered by events;
+// without it the launch is a lone case's, dependent on the one before it.  PUSH: stores also go to the
 // neighbour slab that keeps the plane as a halo plane.
 template <bool STAGE2, bool PERSISTENT, bool RANGE = false, bool PUSH = false>
-__device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, const CUtensorMap* tmC,
-                                           const StageArgs& a, const float* __restrict__ Bp,
-                                           float* __restrict__ Outp, int bx, int by, int bz, int kz) {
+__device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const StageArgs& a, const float* __restrict__ Bp, float* __restrict__ Outp, int bx, int by, int bz,
+                                           int kz) {
   const int t = threadIdx.x, tx2 = t & 15, ty = t >> 4;
   const int i0 = bx * TX, j0 = by * TY;
   const int x0 = i0 + 2 * tx2, j = j0 + ty;
@@ -354,6 +389,8 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
   else if (t < 96) { hp_y = 2 + (t & 15); hp_p = (t & 16) ? TX / 2 + 1 : 0; }
   const int hp_x = i0 - 2 + 2 * hp_p, hp_j = j0 + hp_y - 2;
 
+  constexpr bool BARE = !PERSISTENT && !RANGE;  // (a persistent kernel's cases carry the halo maps only)
+  auto outer = [&](int p) { return BARE && (p < k0 || p >= k1); };
   if (PERSISTENT) __syncthreads();  // a previous tile of this CTA is completely done with the shared memory
   if (t == 0) {
     for (int s = 0; s < NSLOT; s++) mbar_init(&S.bar[s], 1);
@@ -367,12 +404,12 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
   }
   if (t == 0) {
     fence_proxy_async_smem();  // earlier tiles' generic reads of the slots before these copies
-    for (int p = k0 - 2; p <= k0 + 1; p++) issue_plane(S, tmQ, tmC, a, p, k0, i0, j0);
+    for (int p = k0 - 2; p <= k0 + 1; p++) issue_plane(S, maps, a, p, k0, outer(p), i0, j0);
   }
   auto own = [&](int kk, f2 P[5]) -> uint32_t {
     const Slot& s = S.slot[slot_of(kk, k0)];
-    if (own_in && kk >= 0 && kk < a.NZ) return slot_pair<true>(a, s, x0, j, kk, i0, j0, P);
-    return slot_pair<false>(a, s, x0, j, kk, i0, j0, P);
+    if (own_in && kk >= 0 && kk < a.NZ) return slot_pair<true>(a, s, x0, j, kk, outer(kk), i0, j0, P);
+    return slot_pair<false>(a, s, x0, j, kk, outer(kk), i0, j0, P);
   };
 
   bool ok = true;
@@ -404,7 +441,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     drain(S, a, k0, first_pending, last_issued);
     return false;
   }
-  if (t == 0) issue_plane(S, tmQ, tmC, a, k0 + 2, k0, i0, j0);
+  if (t == 0) issue_plane(S, maps, a, k0 + 2, k0, outer(k0 + 2), i0, j0);
   last_issued = k0 + 2;
 
   for (int k = k0; k < k1; k++) {
@@ -418,8 +455,8 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     if (t < 96) {
       f2 P[5];
       const bool inside = tile_in && k >= 0 && k < a.NZ;
-      const uint32_t c = inside ? slot_pair<true>(a, S.slot[sk], hp_x, hp_j, k, i0, j0, P)
-                                : slot_pair<false>(a, S.slot[sk], hp_x, hp_j, k, i0, j0, P);
+      const uint32_t c = inside ? slot_pair<true>(a, S.slot[sk], hp_x, hp_j, k, false, i0, j0, P)
+                                : slot_pair<false>(a, S.slot[sk], hp_x, hp_j, k, false, i0, j0, P);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.P[v][hp_y][hp_p] = P[v];
       S.C[hp_y][hp_p] = (uint16_t)c;
@@ -428,7 +465,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const CUtensorMap* tmQ, 
     if (k + 3 <= k1 + 1) {
       if (t == 0) {
         fence_proxy_async_smem();
-        issue_plane(S, tmQ, tmC, a, k + 3, k0, i0, j0);
+        issue_plane(S, maps, a, k + 3, k0, outer(k + 3), i0, j0);
       }
       last_issued = k + 3;
     }
