@@ -13,22 +13,30 @@ using namespace pair;
 // At most 128 registers: two CTAs (16 warps) per SM.  MODE 0: all planes of a lone case, dependent on
 // the launch before; 1: planes [a.kb, a.ke) (a z chunk, a slab's own planes, a case of a batch); 2: the
 // same with the halo push of a z slab.
-template <bool STAGE2, int MODE>
+template <bool STAGE2, int MODE, int ORDER>
 __global__ void __launch_bounds__(NT, 2)
     k_stage_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmQo, const __grid_constant__ CUtensorMap tmCo, StageArgs a,
                  int kz) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   PairSmem& S = *reinterpret_cast<PairSmem*>(smem_raw);
-  stage_tile<STAGE2, false, MODE >= 1, MODE == 2>(S, Maps{&tmQ, &tmC, &tmQo, &tmCo}, a, a.B, a.Out, blockIdx.x,
+  stage_tile<STAGE2, false, MODE >= 1, MODE == 2, ORDER>(S, Maps{&tmQ, &tmC, &tmQo, &tmCo}, a, a.B, a.Out, blockIdx.x,
                                                   blockIdx.y, blockIdx.z, kz);
 }
 
-template <bool STAGE2, int MODE>
-int set_attributes() {
-  A3D_CUDA(cudaFuncSetAttribute(k_stage_pair<STAGE2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <bool STAGE2, int MODE, int ORDER>
+int set_attributes_of() {
+  A3D_CUDA(cudaFuncSetAttribute(k_stage_pair<STAGE2, MODE, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)pair_smem_bytes()));
-  A3D_CUDA(cudaFuncSetAttribute(k_stage_pair<STAGE2, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  A3D_CUDA(cudaFuncSetAttribute(k_stage_pair<STAGE2, MODE, ORDER>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  return A3D_OK;
+}
+template <int MODE>
+int set_attributes() {
+  A3D_TRY((set_attributes_of<false, MODE, 1>()));
+  A3D_TRY((set_attributes_of<true, MODE, 1>()));
+  A3D_TRY((set_attributes_of<false, MODE, 2>()));
+  A3D_TRY((set_attributes_of<true, MODE, 2>()));
   return A3D_OK;
 }
 
@@ -45,10 +53,9 @@ void launch_mode(const a3d_solver* s, const StageArgs& a, int qin_buf, bool stag
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = dependent ? 1 : 0;
-  if (stage2) cudaLaunchKernelEx(&cfg, k_stage_pair<true, MODE>, s->tmQp[qin_buf], s->tmCp, s->tmQo[qin_buf], s->tmCo, a,
-                                   s->march_kz);
-  else cudaLaunchKernelEx(&cfg, k_stage_pair<false, MODE>, s->tmQp[qin_buf], s->tmCp, s->tmQo[qin_buf], s->tmCo, a,
-                                   s->march_kz);
+  auto k = a.order2 ? (stage2 ? k_stage_pair<true, MODE, 2> : k_stage_pair<false, MODE, 2>)
+                    : (stage2 ? k_stage_pair<true, MODE, 1> : k_stage_pair<false, MODE, 1>);
+  cudaLaunchKernelEx(&cfg, k, s->tmQp[qin_buf], s->tmCp, s->tmQo[qin_buf], s->tmCo, a, s->march_kz);
 }
 
 }  // namespace
@@ -63,8 +70,8 @@ int pair_resident_ctas(int* n) {
   int dev = 0, sms = 0, per_sm = 0;
   A3D_CUDA(cudaGetDevice(&dev));
   A3D_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  A3D_TRY((set_attributes<false, 1>()));
-  A3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pair<false, 1>, NT, pair_smem_bytes()));
+  A3D_TRY((set_attributes_of<false, 1, 2>()));
+  A3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pair<false, 1, 2>, NT, pair_smem_bytes()));
   *n = sms * std::max(1, per_sm);
   return A3D_OK;
 }
@@ -98,12 +105,9 @@ int make_pair_tensor_maps(a3d_solver* s) {
     r = enc(&s->tmCo, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, s->code, cd, cs, bare, ce, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(pair codes) failed: %d", (int)r); return A3D_ERR_CUDA; }
-  A3D_TRY((set_attributes<false, 0>()));
-  A3D_TRY((set_attributes<true, 0>()));
-  A3D_TRY((set_attributes<false, 1>()));
-  A3D_TRY((set_attributes<true, 1>()));
-  A3D_TRY((set_attributes<false, 2>()));
-  A3D_TRY((set_attributes<true, 2>()));
+  A3D_TRY(set_attributes<0>());
+  A3D_TRY(set_attributes<1>());
+  A3D_TRY(set_attributes<2>());
   return A3D_OK;
 }
 

@@ -14,7 +14,7 @@
 // source, baffles - stands behind one test of the pair's codes.  9009 warp instructions per plane
 // of a tile in stage 1 (9712 with the apertures carried through shared memory and the wall term
 // formed for every cell); fighter 4.13M cells 17.05 -> 18.7 G cell-updates/s, airliner 120M 19.9 ->
-// 22.3.  The loop must also fit the instruction caches: unrolled by two planes, which removes the
+// 22.3 (22.6 with the order of the scheme a constant).  The loop must also fit the instruction caches: unrolled by two planes, which removes the
 // 42 register moves a plane and pair, it is 37 KB long and measured 18.0 at 120M.
 //
 // The planes arrive through a 4-deep ring of shared-memory slots filled by
@@ -197,6 +197,7 @@ __device__ __forceinline__ void weigh(uint32_t c, const float* ap, int q, f2 G[5
 // (cells x0, x0+1 of row jj, plane k).  c: the pair's primitives; cl, cc: codes of the pair to
 // the left and of this pair.  The slopes of cells x0-1, x0, x0+1 are each formed once.
 // G: aperture-weighted fluxes (mass, x-, y-, z-momentum, energy).
+template <int ORDER>
 __device__ __forceinline__ void xfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cl,
                                      uint32_t cc, int q, uint32_t okm, f2 G[5]) {
   const float h1 = half_if((cl >> 8) & okm, C_OKX), h2 = half_if(cc & okm, C_OKX);
@@ -204,6 +205,11 @@ __device__ __forceinline__ void xfaces(const StageArgs& a, const PairSmem& S, in
   f2 Ls[5], Rs[5];
 #pragma unroll
   for (int v = 0; v < 5; v++) {
+    if (ORDER == 1) {
+      Ls[v] = make_float2(S.P[v][y][p - 1].y, c[v].x);
+      Rs[v] = c[v];
+      continue;
+    }
     const f2 ab = S.P[v][y][p - 1];   // cells x0-2, x0-1
     const float e = S.P[v][y][p + 1].x;  // cell x0+2
     const float p0 = ab.x, p1 = ab.y, p2 = c[v].x, p3 = c[v].y;
@@ -227,6 +233,7 @@ __device__ __forceinline__ void xfaces(const StageArgs& a, const PairSmem& S, in
 
 // y faces j-1/2 of the two cells (x0, x0+1) at plane-array pair p, row y (cell row jj, plane
 // k).  c: their primitives; cb, cc: codes of the pair in row y-1 and of this pair.
+template <int ORDER>
 __device__ __forceinline__ void yfaces(const StageArgs& a, const PairSmem& S, int y, int p, const f2 c[5], uint32_t cb,
                                      uint32_t cc, int qb, uint32_t okm, f2 G[5]) {
   const f2 hL = make_float2(half_if(cb & okm, C_OKY), half_if(cb & okm, C_OKY << 8));
@@ -234,6 +241,11 @@ __device__ __forceinline__ void yfaces(const StageArgs& a, const PairSmem& S, in
   f2 Ls[5], Rs[5];
 #pragma unroll
   for (int v = 0; v < 5; v++) {
+    if (ORDER == 1) {
+      Ls[v] = S.P[v][y - 1][p];
+      Rs[v] = c[v];
+      continue;
+    }
     const f2 pa = S.P[v][y - 2][p], pb = S.P[v][y - 1][p], pe = S.P[v][y + 1][p];
     const f2 d1 = sub(pb, pa), d2 = sub(c[v], pb), d3 = sub(pe, c[v]);
     const f2 sL = make_float2(minmod(d1.x, d2.x), minmod(d1.y, d2.y));
@@ -253,6 +265,7 @@ __device__ __forceinline__ void yfaces(const StageArgs& a, const PairSmem& S, in
 // cc), with e (plane k+2, Pe) above.  Lb is b's +z face state, carried from the face below;
 // c's slope gives this face's right state and, in Lc, the left state of the face above: each
 // z slope is formed once.  qb: geometry index of b's first cell.
+template <int ORDER>
 __device__ __forceinline__ void zfaces(const StageArgs& a, const f2 Lb[5], const f2 Pb[5], const f2 Pc[5],
                                      const f2 Pe[5], uint32_t cb, uint32_t cc, int qb, uint32_t okm, f2 G[5],
                                      f2 Lc[5]) {
@@ -261,6 +274,10 @@ __device__ __forceinline__ void zfaces(const StageArgs& a, const f2 Lb[5], const
   f2 Rc[5];
 #pragma unroll
   for (int v = 0; v < 5; v++) {
+    if (ORDER == 1) {
+      Rc[v] = Lc[v] = Pc[v];
+      continue;
+    }
     const f2 d1 = sub(Pc[v], Pb[v]), d2 = sub(Pe[v], Pc[v]);
     const f2 s = make_float2(minmod(d1.x, d2.x), minmod(d1.y, d2.y));
     Rc[v] = fma(hn, s, Pc[v]);
@@ -360,9 +377,13 @@ __device__ __forceinline__ void store_pair(const StageArgs& a, float* __restrict
 // PERSISTENT: the CTA runs further tiles after this one, so the tile starts with a barrier and
 // retires its ring barriers at the end.  RANGE: the z runs cover planes [a.kb, a.ke) only (a z
 // slab's own planes, one z chunk of a pipelined step, a case of a batch), ordered by events;
-// without it the launch is a lone case's, dependent on the one before it.  PUSH: stores also go to the
+// without it the launch is a lone case's, dependent on the one before it.
+// ORDER: 1 or 2 where the order of the scheme is the kernel's, 0 where it comes with the arguments.
+// First order needs no slopes, which were formed and multiplied by 0: us per iteration at first order
+// with the order in the arguments / in the kernel 31k 16.8 / 14.6, 0.39M 42.8 / 37.0, 4.1M 227 / 181,
+// 120M 5398 / 4182 (28.7 G cell-updates/s); at second order, by the constant alone, 120M 5397 / 5326.  PUSH: stores also go to the
 // neighbour slab that keeps the plane as a halo plane.
-template <bool STAGE2, bool PERSISTENT, bool RANGE = false, bool PUSH = false>
+template <bool STAGE2, bool PERSISTENT, bool RANGE = false, bool PUSH = false, int ORDER = 0>
 __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const StageArgs& a, const float* __restrict__ Bp, float* __restrict__ Outp, int bx, int by, int bz,
                                            int kz) {
   const int t = threadIdx.x, tx2 = t & 15, ty = t >> 4;
@@ -378,7 +399,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
   const int NXY = a.NX * a.NY, PL = a.NY * a.NXp;  // plane strides of the geometry and state arrays
   const int q0 = j * a.NX + x0, qp0 = j * a.NXp + x0;  // this pair's indices in plane 0
   const long Np = a.Np;
-  const uint32_t okm = a.order2 ? 0xFFFFu : 0u;  // slope flags count only at second order
+  const uint32_t okm = ORDER == 2 || (ORDER == 0 && a.order2) ? 0xFFFFu : 0u;  // slope flags count only at second order
   const f2 rx = make_float2(in0 ? a.rXd[x0] : 0.f, in1 ? a.rXd[x0 + 1] : 0.f);
   const f2 ry = f2s(jin ? a.rYd[j] : 0.f);
   // halo pair converted by threads 0..95: rows j0-2, j0-1 (warp 0), j0+TY, j0+TY+1 (warp 1),
@@ -429,9 +450,9 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
 #pragma unroll
     for (int v = 0; v < 5; v++) {
       const f2 d1 = sub(Wm[v], Wa[v]), d2 = sub(W0[v], Wm[v]);
-      Lm[v] = fma(hm, make_float2(minmod(d1.x, d2.x), minmod(d1.y, d2.y)), Wm[v]);
+      Lm[v] = ORDER == 1 ? Wm[v] : fma(hm, make_float2(minmod(d1.x, d2.x), minmod(d1.y, d2.y)), Wm[v]);
     }
-    zfaces(a, Lm, Wm, W0, W1, cm, c0, (k0 - 1) * NXY + q0, okm, Gz, Lz);
+    zfaces<ORDER>(a, Lm, Wm, W0, W1, cm, c0, (k0 - 1) * NXY + q0, okm, Gz, Lz);
   }
   if (!ok) S.abort = 1;
   __syncthreads();  // slots of planes k0-2 and k0-1 are free again
@@ -475,13 +496,13 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
     if (c0 & (C_IRR << 8)) ph.y = __ldg(a.phi + q + 1);
     {
       f2 G[5];
-      xfaces(a, S, hy, pp, W0, S.C[hy][pp - 1], c0, q, okm, G);
+      xfaces<ORDER>(a, S, hy, pp, W0, S.C[hy][pp - 1], c0, q, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fx[v][ty][tx2] = G[v];
     }
     {
       f2 G[5];
-      yfaces(a, S, hy, pp, W0, S.C[hy - 1][pp], c0, q - a.NX, okm, G);
+      yfaces<ORDER>(a, S, hy, pp, W0, S.C[hy - 1][pp], c0, q - a.NX, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fy[v][ty][tx2] = G[v];
     }
@@ -490,7 +511,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
       f2 c[5], G[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) c[v] = S.P[v][TY + 2][e + 1];
-      yfaces(a, S, TY + 2, e + 1, c, S.C[TY + 1][e + 1], S.C[TY + 2][e + 1],
+      yfaces<ORDER>(a, S, TY + 2, e + 1, c, S.C[TY + 1][e + 1], S.C[TY + 2][e + 1],
                           k * NXY + (j0 + TY - 1) * a.NX + i0 + 2 * e, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fy[v][TY][e] = G[v];
@@ -499,7 +520,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
       f2 c[5], G[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) c[v] = S.P[v][r + 2][TX / 2 + 1];
-      xfaces(a, S, r + 2, TX / 2 + 1, c, S.C[r + 2][TX / 2], S.C[r + 2][TX / 2 + 1],
+      xfaces<ORDER>(a, S, r + 2, TX / 2 + 1, c, S.C[r + 2][TX / 2], S.C[r + 2][TX / 2 + 1],
                           k * NXY + (j0 + r) * a.NX + i0 + TX, okm, G);
 #pragma unroll
       for (int v = 0; v < 5; v++) S.Fx[v][r][TX / 2] = G[v];
@@ -517,7 +538,7 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
     if (!ok) S.abort = 1;
     f2 W2[5], Gn[5], Ln[5];
     const uint32_t c2 = own(k + 2, W2);
-    zfaces(a, Lz, W0, W1, W2, c0, c1, q, okm, Gn, Ln);
+    zfaces<ORDER>(a, Lz, W0, W1, W2, c0, c1, q, okm, Gn, Ln);
     __syncthreads();
     if (S.abort) { first_pending = k + 2; break; }  // the wait for plane k+2 ran out
     // ---- [C] residual and RK update ----

@@ -166,6 +166,26 @@ def test_automatic_runs_and_chunks_leave_the_bits(aero, cells):
     assert np.array_equal(a.read_array(), b.read_array())
 
 
+@pytest.mark.parametrize("cells,kz,chunks", [(30000, 1, 1), (60000, 3, 1), (60000, 5, 3), (1000000, 0, 0)])
+def test_first_order_tile_matches_the_single_cell_tile(aero, cells, kz, chunks):
+    """The paired tile's own first-order kernels, as one launch a stage and as z chunks, against the
+    single-cell tile, whose order comes with the arguments: the same float32 terms summed in another
+    order, within the two tiles' 4e-6 after 20 iterations, and not the second-order state."""
+    sh = aero.shape_of(aero.build_aircraft("interceptor"))
+    out = []
+    for kernel, order in ((4, 1), (2, 1), (4, 2)):
+        _, s = gpu_case(aero, sh, cells, 1.0, kernel=kernel)
+        if kz and kernel == 4:
+            s.set_kernel(4, kz)
+            s.set_chunks(chunks)
+        s.set_opt(order=order)
+        s.step(20)
+        out.append(s.read_array())
+    a, b, c = out
+    assert max(rel_max_diff(a[v], b[v]) for v in range(5)) < 4e-6
+    assert max(rel_max_diff(a[v], c[v]) for v in range(5)) > 1e-4
+
+
 @pytest.mark.parametrize("kernel", [2, 4])
 def test_bounded_wait_runs_out_reports_timeout_and_recovers(aero, kernel):
     """The TMA tiles' bounded waits (SURVEY failure detection): with the wait limit at 0 every wait
