@@ -494,7 +494,7 @@ extern "C" int a3d_batch_sync(a3d_batch* b) {
   if (rec[0]) {
     // clear the record (the queues were reset by the launches themselves) and report; the
     // failed case keeps its own flag, so its solver reports the timeout until it is rebuilt
-    A3D_CUDA(cudaMemset(b->d_err, 0, sizeof(rec)));
+    A3D_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(rec), b->st));  // before the next step's launches
     const int row = (int)rec[1];
     const a3d_solver* s = b->solvers[b->order[row]];
     set_error("batch stage: a bounded wait ran out in case %d (%dx%dx%d cells), tile %lld, after %lld tiles on "

@@ -429,14 +429,13 @@ extern "C" int a3d_geom_build(const a3d_shape* shape, const int32_t dims[3], con
   A3D_ARG(shape && dims && xf && yf && zf, "null pointer");
   A3D_ARG(dims[0] >= 1 && dims[1] >= 2 && dims[2] >= 1, "grid dims (NY >= 2 for the symmetry mirror)");
   A3D_TRY(use_device(-1));
-  GridDev gd;
-  A3D_TRY(grid_upload(dims, xf, yf, zf, nullptr, gd));
   const long N = (long)dims[0] * dims[1] * dims[2];
+  GridDev gd;
   GeomDev g{};
-  int rc = A3D_OK;
   cudaStream_t st = nullptr;
-  if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) { grid_free(gd); set_error("cudaStreamCreate failed"); return A3D_ERR_CUDA; }
-  rc = geom_alloc(N, g);
+  A3D_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  int rc = grid_upload(dims, xf, yf, zf, st, gd);
+  if (rc == A3D_OK) rc = geom_alloc(N, g);
   if (rc == A3D_OK) rc = geom_build_device(*shape, gd, h, delta_deg, g, st, counts, vol);
   if (rc == A3D_OK) {
     cudaError_t e = cudaSuccess;
@@ -448,6 +447,7 @@ extern "C" int a3d_geom_build(const a3d_shape* shape, const int32_t dims[3], con
     if (ap3 && e == cudaSuccess) e = cudaMemcpy(ap3, g.ap3, N * 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) { set_error("geometry copy-out: %s", cudaGetErrorString(e)); rc = A3D_ERR_CUDA; }
   }
+  cudaStreamSynchronize(st);  // (after an error too: the grid may still be on its way up)
   geom_free(g);
   grid_free(gd);
   cudaStreamDestroy(st);

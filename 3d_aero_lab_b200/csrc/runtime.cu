@@ -275,8 +275,9 @@ int grid_upload(const int32_t dims[3], const double* xf, const double* yf, const
     float* rec = (float*)&h[offs[9 + a]];
     for (int i = 0; i < n[a]; i++) rec[i] = 1.0f / (*hd[a])[i];
   }
-  A3D_CUDA(cudaMemcpy(base, h.data(), off, cudaMemcpyHostToDevice));
-  (void)st;
+  // on the stream of the kernels that read it: a copy from pageable memory returns once the source
+  // is staged, which may be before it has reached the device
+  A3D_CUDA(cudaMemcpyAsync(base, h.data(), off, cudaMemcpyHostToDevice, st));
   return A3D_OK;
 }
 

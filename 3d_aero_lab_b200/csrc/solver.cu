@@ -362,12 +362,11 @@ extern "C" int a3d_solver_create(const int32_t dims[3], const double* xf, const 
   A3D_TRY(new_solver(device, dims, xf, yf, zf, &s));
   const long N = s->N;
   int rc = A3D_OK;
-  cudaError_t e = cudaMemcpy(s->geo.t, t, N, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->geo.phi, phi, N * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->geo.ap0, ap0, N * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->geo.ap1, ap1, N * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->geo.ap2, ap2, N * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(s->geo.ap3, ap3, N * 4, cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(s->geo.t, t, N, cudaMemcpyHostToDevice, s->st);
+  const float* src[5] = {phi, ap0, ap1, ap2, ap3};
+  float* dst[5] = {s->geo.phi, s->geo.ap0, s->geo.ap1, s->geo.ap2, s->geo.ap3};
+  for (int a = 0; a < 5 && e == cudaSuccess; a++)
+    e = cudaMemcpyAsync(dst[a], src[a], N * sizeof(float), cudaMemcpyHostToDevice, s->st);
   if (e != cudaSuccess) { set_error("geometry upload: %s", cudaGetErrorString(e)); rc = A3D_ERR_CUDA; }
   if (rc == A3D_OK) rc = solver_finish_setup(s);
   if (rc != A3D_OK) { a3d_solver_destroy(s); return rc; }
@@ -420,6 +419,7 @@ extern "C" int a3d_solver_create_shape_slab(const a3d_shape* shape, const int32_
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
     if (e != cudaSuccess) { set_error("slab geometry: %s", cudaGetErrorString(e)); rc = A3D_ERR_CUDA; }
   }
+  cudaStreamSynchronize(s->st);  // (after an error too: the full grid may still be on its way up)
   geom_free(full);
   grid_free(gfull);
   if (rc == A3D_OK) rc = solver_finish_setup(s);

@@ -1,0 +1,66 @@
+"""The library's host side - memory, streams, the order of its copies and launches - on a CUDA runtime
+that only keeps a log (fake_cudart.cpp, preloaded into a child process).  No GPU."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_INCLUDE = "/usr/local/cuda/include"
+
+PRELUDE = """
+import ctypes as C, importlib, sys
+import numpy as np
+sys.path.insert(0, %r)
+fake = C.CDLL(None)
+fake.fake_log.restype = C.c_char_p
+fake.fake_live.restype = C.c_long
+fake.fake_set.argtypes = [C.c_char_p, C.c_long]
+def log():
+    return [line.split() for line in fake.fake_log().decode().splitlines()]
+aero = importlib.import_module("3d_aero_lab_b200")
+cfd = importlib.import_module("3d_aero_lab_b200.cfd")
+L = importlib.import_module("3d_aero_lab_b200._lib")
+lib = L.lib()
+def box(NX, NY, NZ, device=0):
+    "A solver over a box of fluid."
+    N = NX * NY * NZ
+    geo = cfd.Geom(N)
+    geo.t[:], geo.phi[:] = 0, 1
+    for d in range(4):
+        geo.ap[d][:] = d < 3
+    f = lambda n: np.arange(n + 1, dtype=np.float64)
+    return aero.CfdGPU(cfd.Grid(f(NX), f(NY), f(NZ)), geo, device=device)
+""" % ROOT
+
+
+@pytest.fixture(scope="session")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", CUDA_INCLUDE, "-o", so,
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp")], check=True)
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code)], capture_output=True, text=True,
+                           env=dict(os.environ, LD_PRELOAD=so), timeout=120)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+@pytest.mark.parametrize("make", ["box(20, 6, 9)", "aero.Case(cells=3000).solver",
+                                  "cfd.cfd_geom(aero.shape_of(aero.build_aircraft('fighter')), "
+                                  "cfd.cfd_grid(aero.shape_of(aero.build_aircraft('fighter')), 3000), 0.0)"])
+def test_uploads_go_down_the_stream_that_reads_them(fake, make):
+    """A copy from pageable memory may return before it has reached the device, so it must be queued on
+    the stream of the kernels that read it; on the default stream nothing orders it before them."""
+    fake(f'''
+    fake.fake_clear()
+    x = {make}
+    L = log()
+    assert ["cudaMemcpy", "1"] not in L                      # no host-to-device copy on the default stream
+    readers = {{l[1] for l in L if l[0] == "launch"}}
+    up = [l for l in L if l[0] == "cudaMemcpyAsync" and l[2] == "1"]
+    assert up and len(readers) == 1 and {{l[1] for l in up}} == readers
+    ''')
