@@ -529,7 +529,11 @@ __device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const 
     if (STAGE2 && in0) {
       const float* p = Bp + qp;
 #pragma unroll
-      for (int c = 0; c < 5; c++, p += Np) bq[c] = __ldg(reinterpret_cast<const float2*>(p));
+      for (int c = 0; c < 5; c++, p += Np) {
+        // a dependent launch is resident while earlier ones still write this buffer: not read-only for it
+        if (BARE) bq[c] = load_cg(reinterpret_cast<const float2*>(p));
+        else bq[c] = __ldg(reinterpret_cast<const float2*>(p));
+      }
     }
     // ---- plane k+2 into the column window; z face k+1/2 ----
     ok = mbar_wait(&S.bar[sk2], parity_of(k + 2, k0), a.wait_limit);

@@ -166,6 +166,25 @@ def test_automatic_runs_and_chunks_leave_the_bits(aero, cells):
     assert np.array_equal(a.read_array(), b.read_array())
 
 
+@pytest.mark.parametrize("cells,order", [(300, 2), (2000, 1), (2000, 2), (30000, 2), (150000, 1)])
+def test_dependent_launches_of_many_iterations_leave_the_bits(aero, cells, order):
+    """Stages queued as dependent launches, of which several are resident at once on a small grid,
+    read what the launches before them wrote: hundreds of iterations queued together against the
+    same iterations waited for one by one, and against launches that the chunk path makes."""
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    out = []
+    for turns, chunks in ((1, 1), (400, 1), (1, 2)):
+        g, s = gpu_case(aero, sh, cells, 1.0)
+        s.set_opt(order=order)
+        s.set_chunks(chunks)
+        for _ in range(turns):
+            s.step(400 // turns)
+            s.sync()
+        out.append(s.read_array())
+    assert np.isfinite(out[0]).all()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
 @pytest.mark.parametrize("cells,kz,chunks", [(30000, 1, 1), (60000, 3, 1), (60000, 5, 3), (1000000, 0, 0)])
 def test_first_order_tile_matches_the_single_cell_tile(aero, cells, kz, chunks):
     """The paired tile's own first-order kernels, as one launch a stage and as z chunks, against the
