@@ -258,6 +258,12 @@ int launch_stage(a3d_solver* s, const StageArgs& a, bool dependent) {
 
 namespace {
 
+// First plane of chunk c of K: chunks are whole z runs, as equal as that allows.
+int chunk_first(const a3d_solver* s, int K, int c) {
+  const int runs = (s->grid.NZ + s->march_kz - 1) / s->march_kz;
+  return std::min(s->grid.NZ, (int)((long)c * runs / K) * s->march_kz);
+}
+
 // Number of pipelined z chunks a3d_solver_step uses: kernels 2 and 4 on a whole case only.
 int chunk_count(const a3d_solver* s) {
   if ((s->kernel != KERNEL_TMA && s->kernel != KERNEL_PAIR) || s->nbr[0] || s->nbr[1] || s->own_k0 != 0 ||
@@ -270,7 +276,16 @@ int chunk_count(const a3d_solver* s) {
   // Three chunks beat four while a chunk is less than a wave of 10-plane runs (us per iteration, 3 / 4:
   // 1.1M 82 / 88, 1.8M 126 / 132, 2.4M 150 / 157; 3.0M 180 / 178, 4.0M 228 / 228, 9.1M 442 / 438)
   const int K = s->chunks_req > 0 ? s->chunks_req : s->N >= 2700000 ? 4 : s->N >= kChunkCells ? 3 : 1;
-  return std::max(1, std::min(K, std::min(runs, (int)kMaxChunks)));
+  // A stage reads two planes beyond its chunk and waits for the chunks beside it only, so a chunk
+  // between two others has at least two planes (single-plane runs of a small grid: fewer chunks).
+  int n = std::min(K, std::min(runs, (int)kMaxChunks));
+  auto narrow = [&] {
+    for (int c = 1; c + 1 < n; c++)
+      if (chunk_first(s, n, c + 1) - chunk_first(s, n, c) < 2) return true;
+    return false;
+  };
+  while (n > 2 && narrow()) n--;
+  return std::max(1, n);
 }
 
 // The streams and events of K z chunks.
@@ -504,13 +519,13 @@ namespace {
 // n iterations with the case cut into K z chunks of whole z runs (so every cell sees the same
 // arithmetic as in one launch).  Chunk c's stage waits for the previous stage of chunks c-1 and
 // c+1 only: a stage reads two planes beyond its chunk and writes inside it, so those are its
-// only producers (read after write) and its only remaining readers (write after read).
+// only producers (read after write) and its only remaining readers (write after read): chunk_count
+// leaves no chunk between two others with a single plane.
 int step_chunked(a3d_solver* s, int n, int K) {
-  const int kz = s->march_kz, NZ = s->grid.NZ, runs = (NZ + kz - 1) / kz;
   int kb[kMaxChunks], ke[kMaxChunks];
   for (int c = 0; c < K; c++) {
-    kb[c] = (c * runs / K) * kz;
-    ke[c] = std::min(NZ, ((c + 1) * runs / K) * kz);
+    kb[c] = chunk_first(s, K, c);
+    ke[c] = chunk_first(s, K, c + 1);
   }
   A3D_TRY(chunk_streams(s, K));  // (there already, unless the caller has set the chunks)
   A3D_CUDA(cudaEventRecord(s->ev_fork, s->st));

@@ -134,6 +134,35 @@ def test_pipelined_z_chunks_are_bit_identical(aero, chunks, kernel):
     assert a.residual(1) == b.residual(1)
 
 
+@pytest.mark.parametrize("NZ", range(3, 9))
+def test_z_chunks_of_a_few_planes_are_bit_identical(aero, NZ):
+    """Single-plane runs of a grid with 3 to 8 planes: as few chunks as keep two planes in each chunk
+    between two others, and the bits of one launch per stage."""
+    rng = np.random.default_rng(NZ)
+    NX, NY = 70, 37
+    bg = BoxGrid(rng, NX, NY, NZ)
+    t, phi, ap = box_geometry(rng, NX, NY, NZ)
+    hgeo = aero.cfd.Geom(bg.N)
+    hgeo.t, hgeo.phi, hgeo.ap = t, phi, ap
+    noise = rng.standard_normal((5, NZ, NY, NX))
+    out = []
+    for chunks in (1, 2, 3, 4):
+        s = aero.CfdGPU(aero.cfd.Grid(bg.xf, bg.yf, bg.zf), hgeo)
+        assert s.kernel() == (4, 1)
+        s.set_chunks(chunks)
+        assert s.chunks() == {1: 1, 2: 2, 3: 3 if NZ > 4 else 2, 4: 4 if NZ > 6 else 3 if NZ > 4 else 2}[chunks]
+        F = freestream(0.7, 4.0)
+        s.setFree(F)
+        s.setFix([F, F, F])
+        s.reset()
+        Q0 = s.read_array() * (1 + 0.02 * noise)
+        s.write(Q0.astype(np.float32))
+        s.step(20)
+        out.append(s.read_array())
+    for o in out[1:]:
+        assert np.array_equal(out[0], o, equal_nan=True)
+
+
 @pytest.mark.parametrize("cells,kz", [(2000, 1), (98000, 1), (150000, 2)])
 def test_automatic_z_run_takes_single_planes_on_one_wave(aero, cells, kz):
     """Kernel 4's automatic z run: single planes where all their CTAs are resident at once, longer

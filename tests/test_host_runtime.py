@@ -64,3 +64,44 @@ def test_uploads_go_down_the_stream_that_reads_them(fake, make):
     up = [l for l in L if l[0] == "cudaMemcpyAsync" and l[2] == "1"]
     assert up and len(readers) == 1 and {{l[1] for l in up}} == readers
     ''')
+
+
+@pytest.mark.parametrize("kernel", [2, 4])
+def test_z_chunks_wait_for_every_chunk_that_they_read(fake, kernel):
+    """Whatever the planes, the z run and the chunks asked for: every earlier stage's launch over a plane
+    within two of a launch's own is ordered before it, by its stream or by the events it waits for."""
+    fake(f"""
+    for NZ in range(1, 14):
+        s = box(6, 4, NZ)
+        for kz in (0, 1, 2, 3):
+            s.set_kernel({kernel}, kz)
+            run = s.kernel()[1]
+            for chunks in (2, 3, 4):
+                s.set_chunks(chunks)
+                K = s.chunks()
+                assert 1 <= K <= chunks
+                assert K == min(2, -(-NZ // run)) or K > 2 or run == 1, (NZ, run, chunks, K)
+                fake.fake_clear()
+                s.step(3)
+                if K == 1:
+                    continue
+                done, events, stages = {{}}, {{}}, []      # launches that a stream, an event comes after
+                for line in log():
+                    if line[0] == "record":
+                        events[line[1]] = set(done.setdefault(line[2], set()))
+                    elif line[0] == "wait":
+                        done.setdefault(line[1], set()).update(events[line[2]])
+                    elif line[0] == "launch":
+                        if not stages or len(stages[-1]) == K:
+                            stages.append([])
+                        first = stages[-1][-1][2] if stages[-1] else 0
+                        me = (len(stages), first, min(NZ, first + int(line[2]) * run))
+                        before = done.setdefault(line[1], set())
+                        for earlier in stages[:-1]:
+                            for e in earlier:
+                                if e[1] < me[2] + 2 and e[2] > me[1] - 2:
+                                    assert e in before, (NZ, run, K, me, e)
+                        stages[-1].append(me)
+                        before.add(me)
+                assert len(stages) == 6 and all(x[-1][2] == NZ for x in stages)
+    """)
