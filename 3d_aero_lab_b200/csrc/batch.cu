@@ -564,11 +564,13 @@ extern "C" int a3d_batch_tune(a3d_batch* b, int32_t trial_iters, int32_t* best_k
   }
   for (int k = 0; k < n; k++) {  // restore
     a3d_solver* s = b->solvers[k];
-    cudaStreamSynchronize(b->st);
+    cudaError_t e = cudaStreamSynchronize(b->st);
     if (saved[k]) {
-      cudaMemcpy(s->buf[s->iQ], saved[k], 5 * s->Np * sizeof(float), cudaMemcpyDeviceToDevice);
-      cudaDeviceSynchronize();
-      dev_free(saved[k]);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s->buf[s->iQ], saved[k], 5 * s->Np * sizeof(float), cudaMemcpyDeviceToDevice, s->st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+      if (e == cudaSuccess) dev_free(saved[k]);
+      else if (rc == A3D_OK) { set_error("tune: %s", cudaGetErrorString(e)); rc = A3D_ERR_CUDA; }
     }
     s->it = saved_it[k];
   }

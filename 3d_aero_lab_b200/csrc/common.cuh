@@ -37,8 +37,8 @@ void clear_error();
 int use_device(int device);
 
 // Device memory of the current device from the library's pool (runtime.cu).  dev_alloc / dev_free:
-// like cudaMalloc and cudaFree, but a block is freed only once no work that uses it is queued on
-// any stream (cudaFree would have waited).  temp_alloc: stream-ordered, freed by cudaFreeAsync.
+// like cudaMalloc and cudaFree, but dev_free does not wait: its caller has made sure that no work
+// that uses the block is queued on any stream.  temp_alloc: stream-ordered, freed by cudaFreeAsync.
 cudaError_t dev_alloc_raw(void** p, size_t bytes);
 void dev_free(void* p);
 cudaError_t temp_alloc_raw(void** p, size_t bytes, cudaStream_t st);
@@ -46,6 +46,8 @@ template <typename T>
 cudaError_t dev_alloc(T** p, size_t bytes) { return dev_alloc_raw((void**)p, bytes); }
 template <typename T>
 cudaError_t temp_alloc(T** p, size_t bytes, cudaStream_t st) { return temp_alloc_raw((void**)p, bytes, st); }
+// Waits for all work queued on the current device (runtime.cu).
+cudaError_t device_wait();
 // Non-blocking streams of the current device, kept for reuse; put back with no work on them.
 cudaError_t stream_get(cudaStream_t* st);
 void stream_put(cudaStream_t st);

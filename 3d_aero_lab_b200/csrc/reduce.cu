@@ -446,10 +446,9 @@ extern "C" int a3d_solver_set_owned(a3d_solver* s, int32_t k0, int32_t k1) {
   A3D_ARG(s, "null solver");
   A3D_ARG(0 <= k0 && k0 < k1 && k1 <= s->grid.NZ, "owned planes must satisfy 0 <= k0 < k1 <= NZ");
   A3D_CUDA(cudaSetDevice(s->device));
-  A3D_CUDA(cudaStreamSynchronize(s->st));
+  A3D_CUDA(cudaStreamSynchronize(s->st));  // (only the solver's own stream reads the list)
   s->own_k0 = k0;
   s->own_k1 = k1;
-  A3D_CUDA(cudaDeviceSynchronize());  // nothing still reads the list
   dev_free(s->fl.block);
   s->fl = ForceList();
   A3D_TRY(build_force_list(s));

@@ -125,6 +125,15 @@ void dev_free(void* p) {
   }
 }
 
+// cudaDeviceSynchronize is refused while any stream of the device is being captured, by another
+// thread too (a batch's graph), and spoils that capture.  Freeing a block of cudaMalloc waits as
+// well, and other threads' captures allow it.
+cudaError_t device_wait() {
+  void* p = nullptr;
+  const cudaError_t e = cudaMalloc(&p, 1);
+  return e == cudaSuccess ? cudaFree(p) : e;
+}
+
 // Streams of the current device; making and destroying one takes 50 us each, a case has up to
 // five.  At most kStreamsKeep idle ones are kept, none once the last one in use comes back.
 cudaError_t stream_get(cudaStream_t* st) {

@@ -443,11 +443,30 @@ extern "C" int a3d_solver_create_shape_slab(const a3d_shape* shape, const int32_
   return A3D_OK;
 }
 
+namespace {
+
+// Waits for all work that may use the solver's memory.  Its own streams come after whatever the
+// library queued elsewhere (batches, plane copies, interpolation: by events); what neighbour slabs
+// store into it, or a caller queued on streams of its own with an address from
+// a3d_solver_plane_ptr, only a wait for the device covers.
+cudaError_t wait_for_users(const a3d_solver* s) {
+  cudaError_t e = s->st ? cudaStreamSynchronize(s->st) : cudaSuccess;
+  for (cudaStream_t c : s->cst)
+    if (c && e == cudaSuccess) e = cudaStreamSynchronize(c);
+  if (s->foreign && e == cudaSuccess) e = device_wait();
+  return e;
+}
+
+}  // namespace
+
 extern "C" int a3d_solver_destroy(a3d_solver* s) {
   if (!s) return A3D_OK;
   cudaSetDevice(s->device);
-  // all work that may use the solver's memory, a caller's on streams of its own included
-  cudaDeviceSynchronize();
+  const cudaError_t e = wait_for_users(s);
+  if (e != cudaSuccess) {  // its memory and streams go to no other solver
+    set_error("the solver's work could not be waited for: %s", cudaGetErrorString(e));
+    return A3D_ERR_CUDA;
+  }
   dev_free(s->state);
   dev_free(s->code);
   dev_free(s->d_red);
@@ -667,6 +686,8 @@ extern "C" int a3d_solver_set_neighbors(a3d_solver* s, a3d_solver* lo, a3d_solve
   }
   if (lo) A3D_ARG(lo->z_lo < s->z_lo, "lower neighbour must start below");
   if (hi) A3D_ARG(hi->z_lo > s->z_lo, "upper neighbour must start above");
+  for (a3d_solver* n : {lo, hi})
+    if (n) n->foreign = true;
   s->nbr[0] = lo;
   s->nbr[1] = hi;
   return A3D_OK;
@@ -732,6 +753,7 @@ extern "C" int a3d_solver_plane_ptr(a3d_solver* s, int32_t which, int32_t c, int
   clear_error();
   A3D_ARG(s && ptr && plane_floats, "null pointer");
   A3D_ARG((which == 0 || which == 1) && c >= 0 && c < 5 && k >= 0 && k < s->grid.NZ, "which, component or plane");
+  s->foreign = true;
   const long plane = (long)s->grid.NY * s->NXp;
   *ptr = state_buffer(s, which) + c * s->Np + k * plane;
   *plane_floats = plane;

@@ -92,6 +92,7 @@ struct a3d_solver {
   int own_k0 = 0, own_k1 = 0;     // own planes: the ones stage kernels store and reductions cover
   int z_lo = 0;                   // global index of the slab's plane 0
   a3d_solver* nbr[2] = {nullptr, nullptr};  // lower/upper neighbour slab the stage kernels push to
+  bool foreign = false;           // work on other streams may use its state unseen (neighbours, a caller)
   cudaEvent_t ev = nullptr;       // orders plane copies and pushes between solvers
   // pipelined z chunks of a3d_solver_step (kernel 2): chunk c's stages run on stream cst[c] and
   // wait only for chunks c-1 and c+1, so one stage's tail overlaps the next stage's start

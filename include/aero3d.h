@@ -125,6 +125,8 @@ int a3d_solver_create(const int32_t dims[3], const double* xf, const double* yf,
 int a3d_solver_create_shape(const a3d_shape* shape, const int32_t dims[3],
                             const double* xf, const double* yf, const double* zf,
                             double h, double delta_deg, int device, a3d_solver** out);
+/* Waits for the solver's work, then frees it.  If the wait fails its status is returned and
+ * nothing is freed.                                                                      */
 int a3d_solver_destroy(a3d_solver* s);
 /* Grid size and the device the solver lives on. */
 int a3d_solver_dims(a3d_solver* s, int32_t dims[3], int64_t* n_cells);
@@ -206,7 +208,8 @@ int a3d_solver_set_wait_limit(a3d_solver* s, uint32_t limit);
 int a3d_solver_set_chunks(a3d_solver* s, int32_t chunks);
 /* The number of chunks (stage launches per RK stage) a3d_solver_step uses for this case.  */
 int a3d_solver_get_chunks(a3d_solver* s, int32_t* chunks);
-/* The solver's CUDA stream (a cudaStream_t), for callers that time or order work on it. */
+/* The solver's CUDA stream (a cudaStream_t), for callers that time or order work on it.  The
+ * handle is the solver's until a3d_solver_destroy; after that it may be another solver's. */
 int a3d_solver_stream(a3d_solver* s, void** stream);
 /* Blocks until all work queued on the solver's stream has finished. */
 int a3d_solver_sync(a3d_solver* s);

@@ -3,6 +3,8 @@ both batch tiles (kernel 2: the TMA tile, kernel 4: the paired-cell tile).  The 
 first z face of a run in their prologue, where the compiler may round one operation
 differently, so a case is bit-identical at equal run length and agrees to float32 rounding
 across run lengths."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -153,4 +155,51 @@ def test_stream_mode_captures_chunked_steps(aero):
     b.sync()
     for a, c in zip(alone, batched):
         assert np.array_equal(c.solver.read_array(), a.solver.read_array())
+    b.dispose()
+
+
+def test_cases_come_and_go_while_another_thread_captures(aero):
+    """One thread steps a batch by odd counts, which captures a new graph every time, while others make,
+    step and drop cases: no error on either side, and the states of the same steps alone."""
+    def mine():
+        return [aero.Case(aircraft_type=c[0], cells=c[1] / 4, M=c[2], alpha=c[3], delta=c[4]) for c in CASES[:3]]
+
+    def small():
+        c = aero.Case(aircraft_type="fighter", cells=9000, M=0.6, alpha=3.0)
+        c.solver.step(7)
+        c.solver.set_owned(1, c.g.NZ - 1)
+        out = c.solver.read_array()
+        c.solver.plane_ptr(0, 0, 0)
+        c.solver.dispose()
+        return out
+
+    alone, batched = mine(), mine()
+    want = small()
+    bad, stop = [], threading.Event()
+
+    def churn():
+        try:
+            while not stop.is_set():
+                if not np.array_equal(small(), want):
+                    bad.append("state")
+        except Exception as e:
+            bad.append(repr(e))
+
+    ts = [threading.Thread(target=churn) for _ in range(3)]
+    for t in ts:
+        t.start()
+    try:
+        b = aero.Batch([c.solver for c in batched])
+        for _ in range(150):
+            b.step(3)
+        b.sync()
+    finally:
+        stop.set()
+        for t in ts:
+            t.join()
+    assert not bad, bad[:3]
+    for a, c in zip(alone, batched):
+        for _ in range(150):
+            a.solver.step(3)
+        assert np.array_equal(a.solver.read_array(), c.solver.read_array())
     b.dispose()

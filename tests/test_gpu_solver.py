@@ -144,7 +144,7 @@ def test_z_chunks_of_a_few_planes_are_bit_identical(aero, NZ):
     t, phi, ap = box_geometry(rng, NX, NY, NZ)
     hgeo = aero.cfd.Geom(bg.N)
     hgeo.t, hgeo.phi, hgeo.ap = t, phi, ap
-    noise = rng.standard_normal((5, NZ, NY, NX))
+    noise = rng.standard_normal((5, bg.N))
     out = []
     for chunks in (1, 2, 3, 4):
         s = aero.CfdGPU(aero.cfd.Grid(bg.xf, bg.yf, bg.zf), hgeo)
@@ -496,6 +496,25 @@ def test_cases_made_and_dropped_by_several_threads_agree(aero):
     for t in ts:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("cells", [9000, 5000000])
+def test_dispose_waits_for_the_callers_work_on_its_state(aero, cells):
+    """A program that has taken the state's address may have work on it on a stream of its own: the
+    solver's memory goes back to its pool (or, of a large case, to the device) only after that."""
+    import torch
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    g, s = gpu_case(aero, sh, cells, 0.0)
+    s.step(2)
+    s.sync()
+    s.plane_ptr(0, 0, 0)
+    mine, done = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(mine):
+        torch.cuda._sleep(200_000_000)  # 0.1 s; it stands for the work and touches nothing
+        done.record()
+    assert not done.query()
+    s.dispose()
+    assert done.query()
 
 
 def test_display_sampling_matches_oracle(aero, ref):

@@ -105,3 +105,51 @@ def test_z_chunks_wait_for_every_chunk_that_they_read(fake, kernel):
                         before.add(me)
                 assert len(stages) == 6 and all(x[-1][2] == NZ for x in stages)
     """)
+
+
+def test_destruction_waits_for_its_own_streams_and_spoils_no_capture(fake):
+    """A device-wide synchronisation is refused while another thread captures a stream of the device, and
+    spoils that capture: destroying a solver, choosing its planes and tuning a batch make none.  The
+    solver's streams are waited for before its memory goes back."""
+    fake("""
+    fake.fake_set(b"capturing", 1)
+    a, b = box(6, 4, 9), box(6, 4, 9)
+    a.set_kernel(4, 2)
+    a.set_chunks(3)
+    a.step(2)
+    a.set_owned(1, 8)
+    a.set_owned(0, 9)
+    t = aero.Batch([a, b])
+    t.tune(2)
+    t.dispose()
+    assert not [l for l in log() if l[0] == "cudaDeviceSynchronize"]
+    fake.fake_clear()
+    own = str(a.stream)
+    a.dispose()
+    L = log()
+    freed = [i for i, l in enumerate(L) if l[0] in ("cudaFree", "cudaFreeAsync")]
+    waited = {l[1] for l in L[:freed[0]] if l[0] == "cudaStreamSynchronize"}
+    assert own in waited and len(waited) == 4            # its own and the chunks'
+    assert not [l for l in L if l[0] == "cudaMalloc"]                # nobody else had its address
+    b.plane_ptr(0, 0, 0)                                             # b's address is out: the device is waited for
+    fake.fake_clear()
+    b.dispose()
+    order = [l[0] for l in log()]
+    assert order.index("cudaMalloc") < order.index("cudaFree") < order.index("cudaFreeAsync")
+    assert not [l for l in log() if l[0] == "cudaDeviceSynchronize"]
+    """)
+
+
+def test_memory_of_a_solver_that_could_not_be_waited_for_is_not_recycled(fake):
+    fake("""
+    s = box(6, 4, 9)
+    mine, live = str(s.stream), fake.fake_live()
+    fake.fake_fail(b"cudaStreamSynchronize", 900)
+    fake.fake_clear()
+    assert lib.a3d_solver_destroy(s._h) != 0 and b"wait" in lib.a3d_last_error()
+    assert fake.fake_live() == live
+    o = box(6, 4, 9)
+    assert str(o.stream) != mine
+    assert lib.a3d_solver_destroy(s._h) == 0                         # later it can be
+    s._h = C.c_void_p()
+    """)
