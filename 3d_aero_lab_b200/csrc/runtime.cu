@@ -59,6 +59,7 @@ struct Pool {
   std::set<void*> large;      // those from cudaMalloc
   std::vector<cudaStream_t> streams;  // free ones
   long streams_out = 0;       // streams in use
+  void* byte = nullptr;       // of device_wait
 };
 
 std::mutex g_pool_mu;
@@ -127,8 +128,16 @@ void dev_free(void* p) {
 
 // cudaDeviceSynchronize is refused while any stream of the device is being captured, by another
 // thread too (a batch's graph), and spoils that capture.  Freeing a block of cudaMalloc waits as
-// well, and other threads' captures allow it.
+// well, and other threads' captures allow it.  A byte that is never freed keeps the 2 MB mapped that
+// such small blocks are cut from: 5 us for the two calls on an idle device, 640 us without it.
 cudaError_t device_wait() {
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pool* pool = nullptr;
+    cudaError_t e = current_pool(&pool);
+    if (e == cudaSuccess && !pool->byte) e = cudaMalloc(&pool->byte, 1);
+    if (e != cudaSuccess) return e;
+  }
   void* p = nullptr;
   const cudaError_t e = cudaMalloc(&p, 1);
   return e == cudaSuccess ? cudaFree(p) : e;
