@@ -81,6 +81,10 @@ cudaError_t current_pool(Pool** out) {
     e = cudaMemPoolCreate(&pool, &props);
     unsigned long long keep = kPoolKeep;
     if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    // a block never waits for what another stream has yet to give back (it would for all that is
+    // queued there, another solver's steps)
+    int wait = 0;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &wait);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p.st, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
       if (pool) cudaMemPoolDestroy(pool);
@@ -94,36 +98,53 @@ cudaError_t current_pool(Pool** out) {
 
 }  // namespace
 
+// Blocks are taken and given back without the lock: cudaMalloc and cudaFree may take milliseconds, or
+// wait for the device.  A block counts as in use from before it is taken, so that no other thread's
+// last dev_free trims the pool under it.
 cudaError_t dev_alloc_raw(void** p, size_t bytes) {
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  Pool* pool = nullptr;
-  cudaError_t e = current_pool(&pool);
-  if (e != cudaSuccess) return e;
-  if (bytes > kPoolBlock) {
-    e = cudaMalloc(p, bytes);
-    if (e == cudaSuccess) pool->large.insert(*p);
-    return e;
+  const bool large = bytes > kPoolBlock;
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pool* q = nullptr;
+    const cudaError_t e = current_pool(&q);
+    if (e != cudaSuccess) return e;
+    pool = q->pool;
+    st = q->st;
+    if (!large) q->blocks++;
   }
-  e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool->pool, pool->st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(pool->st);
-  if (e == cudaSuccess) pool->blocks++;
+  cudaError_t e;
+  if (large) {
+    e = cudaMalloc(p, bytes);
+  } else {
+    e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  Pool* q = nullptr;
+  if (current_pool(&q) != cudaSuccess) return e;
+  if (e == cudaSuccess && large) q->large.insert(*p);
+  if (e != cudaSuccess && !large) q->blocks--;
   return e;
 }
 
 void dev_free(void* p) {
   if (!p) return;
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  Pool* pool = nullptr;
-  if (current_pool(&pool) != cudaSuccess) return;
-  if (pool->large.erase(p)) {
-    cudaFree(p);
-    return;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pool* pool = nullptr;
+    if (current_pool(&pool) != cudaSuccess) return;
+    if (!pool->large.erase(p)) {
+      cudaFreeAsync(p, pool->st);
+      if (--pool->blocks == 0) {
+        cudaStreamSynchronize(pool->st);
+        cudaMemPoolTrimTo(pool->pool, 0);
+      }
+      return;
+    }
   }
-  cudaFreeAsync(p, pool->st);
-  if (--pool->blocks == 0) {
-    cudaStreamSynchronize(pool->st);
-    cudaMemPoolTrimTo(pool->pool, 0);
-  }
+  cudaFree(p);
 }
 
 // cudaDeviceSynchronize is refused while any stream of the device is being captured, by another

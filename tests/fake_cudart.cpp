@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <unistd.h>
 
 namespace {
 
@@ -19,7 +20,7 @@ struct Call { dim3 grid, block; size_t smem; cudaStream_t st; };
 std::recursive_mutex mu;
 std::string text;
 std::map<std::string, int> fail;        // function -> status of its next call
-std::map<std::string, long> knob = {{"limit", 1L << 50}, {"capturing", 0}};
+std::map<std::string, long> knob = {{"limit", 1L << 50}, {"capturing", 0}, {"free_us", 0}};
 std::map<void*, Block> live;
 std::map<const void*, std::string> names;  // kernels
 size_t in_use = 0, idle[64] = {};
@@ -143,7 +144,11 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 
 // ---- memory
 cudaError_t cudaMalloc(void** p, size_t n) { LOGGED("cudaMalloc", "%zu", n); return take(p, n, -1); }
-cudaError_t cudaFree(void* p) { LOGGED("cudaFree", "%p", p); return give(p); }
+cudaError_t cudaFree(void* p) {
+  LOGGED("cudaFree", "%p", p);
+  if (p) usleep(knob["free_us"]);  // (as if work on the device had to end first)
+  return give(p);
+}
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) { *p = (cudaMemPool_t)(++pools); return cudaSuccess; }

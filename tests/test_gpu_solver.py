@@ -498,6 +498,32 @@ def test_cases_made_and_dropped_by_several_threads_agree(aero):
     assert not bad
 
 
+def test_making_a_case_does_not_wait_for_another_solvers_queue(aero):
+    """Memory that another solver's queue still has to give back is left alone: a case is made while a
+    long queue, with temporary blocks of its own at the end, is far from done."""
+    import torch
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    _, coarse = gpu_case(aero, sh, 300000, 0.0)
+    _, fine = gpu_case(aero, sh, 60000, 0.0)
+    gpu_case(aero, sh, 9000, 0.0)[1].step(1)  # (loads the kernels)
+    fine.interp_from(coarse)
+    fine.sync()
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(torch.cuda.ExternalStream(fine.stream)):
+        torch.cuda._sleep(2_000_000_000)  # 1 s
+    for _ in range(6):
+        fine.interp_from(coarse)
+    with torch.cuda.stream(torch.cuda.ExternalStream(fine.stream)):
+        done.record()
+    made = [gpu_case(aero, sh, c, 0.0)[1] for c in (9000, 12000, 30000, 5000)]
+    for s in made:
+        s.step(2)
+        s.sample(np.array([[1.0, 0.5, 0.2]]))
+    assert not done.query()
+    fine.sync()
+
+
 @pytest.mark.parametrize("cells", [9000, 5000000])
 def test_dispose_waits_for_the_callers_work_on_its_state(aero, cells):
     """A program that has taken the state's address may have work on it on a stream of its own: the

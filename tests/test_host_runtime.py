@@ -153,3 +153,24 @@ def test_memory_of_a_solver_that_could_not_be_waited_for_is_not_recycled(fake):
     assert lib.a3d_solver_destroy(s._h) == 0                         # later it can be
     s._h = C.c_void_p()
     """)
+
+
+def test_a_block_waits_for_no_other_solver(fake):
+    """The pool does not hand out memory that another stream has yet to give back, and a thread that frees
+    a large case, which waits for the device, holds up no other thread's case."""
+    fake("""
+    import threading, time
+    big = box(600, 200, 40)                                          # 288 MB of state: of cudaMalloc
+    a = [l for l in log() if l[0] == "cudaMemPoolSetAttribute"]
+    REUSE_ALLOW_INTERNAL_DEPENDENCIES = 3
+    assert [l[3] for l in a if int(l[2]) == REUSE_ALLOW_INTERNAL_DEPENDENCIES] == ["0"]
+    fake.fake_set(b"free_us", 2000000)
+    t = threading.Thread(target=big.dispose)
+    t.start()
+    time.sleep(0.3)
+    t0 = time.time()
+    small = box(6, 4, 9)
+    assert time.time() - t0 < 1 and t.is_alive()
+    t.join()
+    fake.fake_set(b"free_us", 0)
+    """)
