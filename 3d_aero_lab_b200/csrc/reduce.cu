@@ -328,11 +328,11 @@ int build_force_list(a3d_solver* s) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   if (e != cudaSuccess) { cudaFreeAsync(d_off, s->st); set_error("force list count: %s", cudaGetErrorString(e)); return A3D_ERR_CUDA; }
   const long tot = (long)s->h_red[0];
-  s->fl.n = tot;
   const size_t n1 = (size_t)std::max(tot, 1L);
   char* blk = nullptr;
   e = dev_alloc(&blk, n1 * (8 + 4 * 8) + 256);
   if (e != cudaSuccess) { cudaFreeAsync(d_off, s->st); set_error("force list alloc: %s", cudaGetErrorString(e)); return A3D_ERR_NOMEM; }
+  s->fl.n = tot;
   s->fl.block = blk;
   s->fl.q = (int64_t*)blk;
   s->fl.cx = (double*)(blk + n1 * 8);

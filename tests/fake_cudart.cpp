@@ -19,8 +19,9 @@ struct Call { dim3 grid, block; size_t smem; cudaStream_t st; };
 
 std::recursive_mutex mu;
 std::string text;
-std::map<std::string, int> fail;        // function -> status of its next call
-std::map<std::string, long> knob = {{"limit", 1L << 50}, {"capturing", 0}, {"free_us", 0}};
+struct Failure { int status, calls; };
+std::map<std::string, Failure> fail;    // function -> status of its `calls`th call from now
+std::map<std::string, long> knob = {{"limit", 1L << 50}, {"capturing", 0}, {"free_us", 0}, {"entries", 0}};
 std::map<void*, Block> live;
 std::map<const void*, std::string> names;  // kernels
 size_t in_use = 0, idle[64] = {};
@@ -37,10 +38,8 @@ cudaError_t log(const char* f, const char* fmt = "", ...) {
   va_end(ap);
   text += std::string(f) + " " + b + "\n";
   auto it = fail.find(f);
-  if (it == fail.end() || !it->second) return cudaSuccess;
-  const int e = it->second;
-  it->second = 0;
-  return (cudaError_t)e;
+  if (it == fail.end() || it->second.calls-- != 1) return cudaSuccess;
+  return (cudaError_t)it->second.status;
 }
 
 template <typename T>
@@ -89,7 +88,7 @@ extern "C" {
 // ---- the test's side
 const char* fake_log() { return text.c_str(); }
 void fake_clear() { text.clear(); }
-void fake_fail(const char* f, int status) { fail[f] = status; }
+void fake_fail(const char* f, int status, int calls) { fail[f] = {status, calls}; }
 void fake_set(const char* k, long v) { knob[k] = v; }
 long fake_live() { return (long)live.size(); }
 
@@ -109,7 +108,8 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* st)
   *g = pushed.grid; *b = pushed.block; *smem = pushed.smem; *(cudaStream_t*)st = pushed.st;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3, void**, size_t, cudaStream_t st) {
+cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3, void** args, size_t, cudaStream_t st) {
+  if (names[f].find("k_fl_count") != std::string::npos) **(double**)args[4] = knob["entries"];
   LOGGED("launch", "%ld %u %s", (long)st, g.z, names[f].c_str());
   return cudaSuccess;
 }

@@ -144,7 +144,7 @@ def test_memory_of_a_solver_that_could_not_be_waited_for_is_not_recycled(fake):
     fake("""
     s = box(6, 4, 9)
     mine, live = str(s.stream), fake.fake_live()
-    fake.fake_fail(b"cudaStreamSynchronize", 900)
+    fake.fake_fail(b"cudaStreamSynchronize", 900, 1)
     fake.fake_clear()
     assert lib.a3d_solver_destroy(s._h) != 0 and b"wait" in lib.a3d_last_error()
     assert fake.fake_live() == live
@@ -173,4 +173,20 @@ def test_a_block_waits_for_no_other_solver(fake):
     assert time.time() - t0 < 1 and t.is_alive()
     t.join()
     fake.fake_set(b"free_us", 0)
+    """)
+
+
+def test_a_force_list_that_found_no_memory_is_empty(fake):
+    """Choosing other planes makes a new list; if there is no memory for it the call says so, and no
+    list is left whose length speaks of cells that it does not have."""
+    fake("""
+    fake.fake_set(b"entries", 40)
+    s = box(6, 4, 9)
+    n = C.c_int64()
+    L.check(lib.a3d_solver_force_list(s._h, C.byref(n), 0, None, None, None, None, None))
+    assert n.value == 40
+    fake.fake_fail(b"cudaMallocFromPoolAsync", 2, 2)                 # the offsets' block, then the list's
+    assert lib.a3d_solver_set_owned(s._h, 1, 8) == 3
+    L.check(lib.a3d_solver_force_list(s._h, C.byref(n), 0, None, None, None, None, None))
+    assert n.value == 0
     """)
