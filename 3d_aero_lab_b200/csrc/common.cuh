@@ -53,6 +53,7 @@ cudaError_t stream_get(cudaStream_t* st);
 void stream_put(cudaStream_t st);
 // Lets device `peer` address the pool of `device` (cudaDeviceEnablePeerAccess does not cover pools).
 cudaError_t pool_peer_access(int device, int peer);
+void pool_share(int device);  // the same for every device that can
 // A small page-locked block of kPinnedBytes.
 constexpr size_t kPinnedBytes = 64 * sizeof(double);
 cudaError_t pinned_alloc(double** p);

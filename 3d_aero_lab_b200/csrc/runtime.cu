@@ -60,6 +60,8 @@ struct Pool {
   std::vector<cudaStream_t> streams;  // free ones
   long streams_out = 0;       // streams in use
   void* byte = nullptr;       // of device_wait
+  std::set<int> peers;        // devices that may address the pool's blocks
+  bool shared = false;        // all that can
 };
 
 std::mutex g_pool_mu;
@@ -207,14 +209,30 @@ cudaError_t temp_alloc_raw(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, st);
 }
 
+// (asked once for each pair: cudaMemPoolSetAccess is no call for every halo exchange)
 cudaError_t pool_peer_access(int device, int peer) {
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (device >= (int)g_pools.size() || !g_pools[device].pool) return cudaSuccess;
+  if (device >= (int)g_pools.size() || !g_pools[device].pool || g_pools[device].peers.count(peer)) return cudaSuccess;
   cudaMemAccessDesc d = {};
   d.location.type = cudaMemLocationTypeDevice;
   d.location.id = peer;
   d.flags = cudaMemAccessFlagsProtReadWrite;
-  return cudaMemPoolSetAccess(g_pools[device].pool, &d, 1);
+  const cudaError_t e = cudaMemPoolSetAccess(g_pools[device].pool, &d, 1);
+  if (e == cudaSuccess) g_pools[device].peers.insert(peer);
+  return e;
+}
+
+void pool_share(int device) {
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (device >= (int)g_pools.size() || g_pools[device].shared) return;
+    g_pools[device].shared = true;
+  }
+  int n = 0, can = 0;
+  if (cudaGetDeviceCount(&n) != cudaSuccess) n = 0;
+  for (int d = 0; d < n; d++)
+    if (d != device && cudaDeviceCanAccessPeer(&can, d, device) == cudaSuccess && can) pool_peer_access(device, d);
+  cudaGetLastError();
 }
 
 // Small page-locked blocks (a solver's reduction results), cut from pages that are given back

@@ -753,6 +753,7 @@ extern "C" int a3d_solver_plane_ptr(a3d_solver* s, int32_t which, int32_t c, int
   clear_error();
   A3D_ARG(s && ptr && plane_floats, "null pointer");
   A3D_ARG((which == 0 || which == 1) && c >= 0 && c < 5 && k >= 0 && k < s->grid.NZ, "which, component or plane");
+  pool_share(s->device);  // as reachable for a caller's peer kernels as memory of cudaMalloc
   s->foreign = true;
   const long plane = (long)s->grid.NY * s->NXp;
   *ptr = state_buffer(s, which) + c * s->Np + k * plane;

@@ -237,7 +237,9 @@ int a3d_solver_stage(a3d_solver* s, int32_t which);
 int a3d_solver_copy_planes(a3d_solver* dst, int32_t dst_k0, a3d_solver* src, int32_t src_k0,
                            int32_t nk, int32_t which);
 /* Device address of plane k of component c (planes of a component are contiguous,
- * plane_floats apart), for exchanges the caller runs on the solver's stream (NCCL).      */
+ * plane_floats apart), for exchanges the caller runs on the solver's stream (NCCL).  Devices
+ * that are peers can address it once the caller has enabled that (cudaDeviceEnablePeerAccess).
+ * States below 256 MB are blocks of a memory pool: cudaIpcGetMemHandle does not export them. */
 int a3d_solver_plane_ptr(a3d_solver* s, int32_t which, int32_t c, int32_t k, void** ptr,
                          int64_t* plane_floats);
 /* Halo push instead of copies: s's stage kernels also store the own planes that its lower

@@ -190,3 +190,21 @@ def test_a_force_list_that_found_no_memory_is_empty(fake):
     L.check(lib.a3d_solver_force_list(s._h, C.byref(n), 0, None, None, None, None, None))
     assert n.value == 0
     """)
+
+
+def test_planes_can_be_reached_from_peer_devices(fake):
+    """cudaDeviceEnablePeerAccess covers memory of cudaMalloc but not of a pool: where a state's address
+    goes out, or another device's slab stores into it, the pool is opened to the peers, once."""
+    fake("""
+    grants = lambda: [l[1:] for l in log() if l[0] == "cudaMemPoolSetAccess"]
+    READ_WRITE = "3"
+    a, b = box(6, 4, 9), box(6, 4, 9)
+    assert grants() == []
+    for s in (a, a, b):
+        s.plane_ptr(0, 0, 0)
+    assert grants() == [["1", "1", READ_WRITE]]                      # device 0's pool to device 1
+    c = box(6, 4, 9, device=1)
+    for _ in range(5):
+        c.copy_planes_from(a, 0, 4, 2, 0)
+    assert sorted(grants()) == [["1", "1", READ_WRITE], ["2", "0", READ_WRITE]]
+    """)
