@@ -65,7 +65,8 @@ struct Pool {
 };
 
 std::mutex g_pool_mu;
-std::vector<Pool> g_pools;  // by device
+// by device; never destroyed: solvers may be, and threads may run, while the process exits
+std::vector<Pool>& g_pools = *new std::vector<Pool>;
 
 // The current device's pool, made at its first use.  Caller holds g_pool_mu.
 cudaError_t current_pool(Pool** out) {
@@ -246,7 +247,7 @@ struct PinnedPage {
   bool taken[kPinnedBlocks] = {};
 };
 std::mutex g_pinned_mu;
-std::vector<PinnedPage> g_pinned;
+std::vector<PinnedPage>& g_pinned = *new std::vector<PinnedPage>;  // (as g_pools)
 
 }  // namespace
 

@@ -17,13 +17,15 @@ namespace {
 struct Block { size_t bytes; int pool; };  // pool -1: of cudaMalloc
 struct Call { dim3 grid, block; size_t smem; cudaStream_t st; };
 
+// (never destroyed: the library may call while the process exits)
 std::recursive_mutex mu;
-std::string text;
+std::string& text = *new std::string;
 struct Failure { int status, calls; };
-std::map<std::string, Failure> fail;    // function -> status of its `calls`th call from now
-std::map<std::string, long> knob = {{"limit", 1L << 50}, {"capturing", 0}, {"free_us", 0}, {"entries", 0}};
-std::map<void*, Block> live;
-std::map<const void*, std::string> names;  // kernels
+std::map<std::string, Failure>& fail = *new std::map<std::string, Failure>;   // function -> status of its `calls`th call from now
+std::map<std::string, long>& knob =
+    *new std::map<std::string, long>{{"limit", 1L << 50}, {"capturing", 0}, {"free_us", 0}, {"entries", 0}};
+std::map<void*, Block>& live = *new std::map<void*, Block>;
+std::map<const void*, std::string>& names = *new std::map<const void*, std::string>;  // kernels
 size_t in_use = 0, idle[64] = {};
 long next_handle = 16, pools = 0;
 thread_local int device = 0;
@@ -81,6 +83,13 @@ cudaError_t give(void* p) {
 
 int encode_nothing(...) { return 0; }
 
+// An exit handler from before the library was loaded, which therefore runs after its destructors.
+int (*at_exit)(void*) = nullptr;
+void* at_exit_arg = nullptr;
+__attribute__((constructor)) void early() {
+  atexit([] { if (at_exit && at_exit(at_exit_arg) != 0) _exit(3); });
+}
+
 }  // namespace
 
 extern "C" {
@@ -90,6 +99,7 @@ const char* fake_log() { return text.c_str(); }
 void fake_clear() { text.clear(); }
 void fake_fail(const char* f, int status, int calls) { fail[f] = {status, calls}; }
 void fake_set(const char* k, long v) { knob[k] = v; }
+void fake_at_exit(int (*f)(void*), void* arg) { at_exit = f; at_exit_arg = arg; }
 long fake_live() { return (long)live.size(); }
 
 // ---- registration and launches

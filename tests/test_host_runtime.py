@@ -44,7 +44,7 @@ def fake(tmp_path_factory):
 
     def run(code):
         r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code)], capture_output=True, text=True,
-                           env=dict(os.environ, LD_PRELOAD=so), timeout=120)
+                           env=dict(os.environ, LD_PRELOAD=so, MALLOC_PERTURB_="165"), timeout=120)
         assert r.returncode == 0, r.stdout + r.stderr
     return run
 
@@ -207,4 +207,15 @@ def test_planes_can_be_reached_from_peer_devices(fake):
     for _ in range(5):
         c.copy_planes_from(a, 0, 4, 2, 0)
     assert sorted(grants()) == [["1", "1", READ_WRITE], ["2", "0", READ_WRITE]]
+    """)
+
+
+@pytest.mark.parametrize("size", ["6, 4, 9", "600, 200, 40"])  # state in the pool, from cudaMalloc
+def test_a_solver_may_be_destroyed_while_the_process_exits(fake, size):
+    """By an exit handler, a global object of the program or a thread that still runs: the pools are
+    there to the end.  (Freed memory is overwritten in these tests, so that its use shows.)"""
+    fake(f"""
+    s = box({size})
+    fake.fake_at_exit(lib.a3d_solver_destroy, s._h)
+    s._h = C.c_void_p()
     """)
