@@ -275,7 +275,11 @@ int chunk_count(const a3d_solver* s) {
   // 58.7 / 60.1, 914k 69.6 / 69.5 and 61.5 / 63.4, 933k 69.7 / 67.4, 1.1M 84.6 / 82.5 and 79.8 / 73.7).
   // Three chunks beat four while a chunk is less than a wave of 10-plane runs (us per iteration, 3 / 4:
   // 1.1M 82 / 88, 1.8M 126 / 132, 2.4M 150 / 157; 3.0M 180 / 178, 4.0M 228 / 228, 9.1M 442 / 438)
-  const int K = s->chunks_req > 0 ? s->chunks_req : s->N >= 2700000 ? 4 : s->N >= kChunkCells ? 3 : 1;
+  // The single-cell tile has no dependent launches: its chunks pay earlier (us per iteration, one
+  // launch / 4 chunks: 825k 84.1 / 70.4, 933k 96.3 / 80.2; 3 / 4: 1.1M 94 / 96, 1.5M 125 / 123, 2.6M 194 / 194).
+  const int automatic = s->kernel == KERNEL_TMA ? (s->N >= 800000 ? 4 : 1)
+                                                : s->N >= 2700000 ? 4 : s->N >= kChunkCells ? 3 : 1;
+  const int K = s->chunks_req > 0 ? s->chunks_req : automatic;
   // A stage reads two planes beyond its chunk and waits for the chunks beside it only, so a chunk
   // between two others has at least two planes (single-plane runs of a small grid: fewer chunks).
   int n = std::min(K, std::min(runs, (int)kMaxChunks));
@@ -580,8 +584,8 @@ int step_chunked(a3d_solver* s, int n, int K) {
 
 }  // namespace
 
-// Pipelined z chunks of a3d_solver_step (kernel 2): 0 = automatic (4 from 2.7M cells up, 3 from 0.95M, else 1),
-// 1 = one launch per stage, 2..4 = that many chunks.  Results do not depend on it.
+// Pipelined z chunks of a3d_solver_step (kernels 2 and 4): 0 = automatic, 1 = one launch per stage, 2..4 = that
+// many chunks, or as many as the planes allow (chunk_count).  Results do not depend on it.
 extern "C" int a3d_solver_set_chunks(a3d_solver* s, int32_t chunks) {
   clear_error();
   A3D_ARG(s, "null solver");

@@ -48,7 +48,7 @@ struct ForceList {
 // Stage kernels by number (the numbers 1 and 3 belonged to two tiles since retired: slower
 // than the TMA tiles on every measured case).
 enum StageKernel { KERNEL_CELL = 0, KERNEL_TMA = 2, KERNEL_PAIR = 4 };
-constexpr long kChunkCells = 950000;  // from here on a step runs as z chunks
+constexpr long kChunkCells = 950000;  // from here on a step on the paired tile runs as z chunks
 constexpr int kMaxChunks = 4;  // z chunks of a pipelined step (6 or 8 measured no faster)
 
 }  // namespace a3d
@@ -94,7 +94,7 @@ struct a3d_solver {
   a3d_solver* nbr[2] = {nullptr, nullptr};  // lower/upper neighbour slab the stage kernels push to
   bool foreign = false;           // work on other streams may use its state unseen (neighbours, a caller)
   cudaEvent_t ev = nullptr;       // orders plane copies and pushes between solvers
-  // pipelined z chunks of a3d_solver_step (kernel 2): chunk c's stages run on stream cst[c] and
+  // pipelined z chunks of a3d_solver_step (kernels 2 and 4): chunk c's stages run on stream cst[c] and
   // wait only for chunks c-1 and c+1, so one stage's tail overlaps the next stage's start
   int chunks_req = 0;             // 0: automatic
   cudaStream_t cst[a3d::kMaxChunks] = {};

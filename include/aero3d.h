@@ -203,8 +203,9 @@ int a3d_solver_get_kernel(a3d_solver* s, int32_t* kernel, int32_t* march_kz);
 int a3d_solver_set_wait_limit(a3d_solver* s, uint32_t limit);
 /* Kernels 2 and 4 step the case as up to 4 z chunks of whole z runs on their own streams, each
  * chunk's stage waiting only for its neighbour chunks' previous stage: the tail of one stage
- * overlaps the start of the next.  0 = automatic (4 chunks from 2.7M cells up, 3 from 0.95M, else 1),
- * 1 = one launch per stage, 2..4 = that many chunks.  The results are the same bit for bit. */
+ * overlaps the start of the next.  0 = automatic (kernel 4: 4 chunks from 2.7M cells up, 3 from
+ * 0.95M, else 1; kernel 2: 4 from 0.8M, else 1), 1 = one launch per stage, 2..4 = that many
+ * chunks (fewer on a grid of a few planes).  The results are the same bit for bit.        */
 int a3d_solver_set_chunks(a3d_solver* s, int32_t chunks);
 /* The number of chunks (stage launches per RK stage) a3d_solver_step uses for this case.  */
 int a3d_solver_get_chunks(a3d_solver* s, int32_t* chunks);

@@ -219,3 +219,15 @@ def test_a_solver_may_be_destroyed_while_the_process_exits(fake, size):
     fake.fake_at_exit(lib.a3d_solver_destroy, s._h)
     s._h = C.c_void_p()
     """)
+
+
+@pytest.mark.parametrize("kernel,NZ,chunks", [(2, 79, 1), (2, 80, 4), (2, 94, 4), (2, 280, 4),
+                                              (4, 80, 1), (4, 94, 1), (4, 95, 3), (4, 269, 3), (4, 270, 4)])
+def test_automatic_chunks_of_each_tile(fake, kernel, NZ, chunks):
+    """Planes of 10,000 cells: the paired tile's dependent launches hold longer than the single-cell
+    tile's plain ones."""
+    fake(f"""
+    s = box(100, 100, {NZ})
+    s.set_kernel({kernel})
+    assert s.chunks() == {chunks}
+    """)
