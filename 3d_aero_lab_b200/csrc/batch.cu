@@ -237,25 +237,35 @@ std::vector<double> signature(const a3d_solver* s) {
 }
 
 // Mode 1: the z run of the cases whose own is automatic (paired tile only, whose results do not
-// depend on the run), 0 to leave them.  A case's own run is short enough to fill the chip alone;
+// depend on the run): *kz, or where that is 0 their own, but at least *least.  A case's own run is short enough to fill the chip alone;
 // beside others it need not be, and each run costs four planes read and a z face formed twice.
 // So: 16 planes where all cases together still launch two waves of CTAs, else 8 or 4 planes where
 // that makes 1.2 waves.  Measured (us per iteration; own runs, 4, 8, 16 planes): 24 cases, 5.1M
 // cells 475, 408, 372, 369 (3.4 waves at 16); 5 cases, 4.4M 322, 301, 281, 280 (2.4); 8 cases, 2.5M
 // 226, 197, 188, 192 (1.5); 12 cases, 1.5M 156, 131, 128, 141 (1.0); 4 cases, 0.57M 66, 60, 73, 98 (0.5).
-int common_run(a3d_batch* b, int* kz) {
+// Smaller batches keep their own runs, single planes only up to 1.8 waves of them: a wave of single
+// planes takes 5.8 us, of two planes 9.2.  us per iteration, single planes / two (waves of single planes):
+// 2 cases of 60k cells 21.2 / 23.5 (1.4), 4 of 30k 26.8 / 27.6 (1.5), 2 of 100k 29.1 / 27.1 (2.2), 8 of 30k
+// 46.3 / 41.3 (3.0), 24 of 12k 79.5 / 70.8 (3.2), 4 of 100k 51.5 / 41.9 (4.4).
+int common_run(a3d_batch* b, int* kz, int* least) {
   *kz = 0;
+  *least = 1;
   if (b->tma_tile) return A3D_OK;
   int resident = 0;
   A3D_TRY(pair_resident_ctas(&resident));
-  for (int run : {16, 8, 4}) {
+  for (int run : {16, 8, 4, 0}) {  // 0: their own
     long ctas = 0;
     for (const a3d_solver* s : b->solvers) {
-      const int r = s->kz_auto ? run : s->march_kz;
+      const int r = s->kz_auto && run ? run : s->march_kz;
       ctas += (long)((s->grid.NX + pair::TX - 1) / pair::TX) * ((s->grid.NY + pair::TY - 1) / pair::TY) *
               ((s->grid.NZ + r - 1) / r);
     }
-    if (ctas * 5 >= (run == 16 ? 10L : 6L) * resident) { *kz = run; break; }
+    if (run == 0) {
+      if (ctas * 5 > 9L * resident) *least = 2;
+    } else if (ctas * 5 >= (run == 16 ? 10L : 6L) * resident) {
+      *kz = run;
+      break;
+    }
   }
   return A3D_OK;
 }
@@ -266,8 +276,8 @@ int common_run(a3d_batch* b, int* kz) {
 int build_stream_graph(a3d_batch* b) {
   if (b->sgraph) cudaGraphExecDestroy(b->sgraph);
   b->sgraph = nullptr;
-  int kz = 0;
-  A3D_TRY(common_run(b, &kz));
+  int kz = 0, least = 1;
+  A3D_TRY(common_run(b, &kz, &least));
   cudaGraph_t g = nullptr;
   A3D_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
   int rc = A3D_OK;
@@ -278,7 +288,7 @@ int build_stream_graph(a3d_batch* b) {
   for (size_t k = 0; k < b->solvers.size() && rc == A3D_OK; k++) {
     a3d_solver* s = b->solvers[k];
     const int own_kz = s->march_kz;
-    if (kz && s->kz_auto) s->march_kz = kz;
+    if (s->kz_auto) s->march_kz = kz ? kz : std::max(own_kz, least);
     cu(cudaStreamWaitEvent(s->st, b->ev_fork, 0));
     int iQ = s->iQ, iB = s->iB;
     const int iS1 = s->iS1;

@@ -231,3 +231,25 @@ def test_automatic_chunks_of_each_tile(fake, kernel, NZ, chunks):
     s.set_kernel({kernel})
     assert s.chunks() == {chunks}
     """)
+
+
+@pytest.mark.parametrize("cases,run", [(1, 1), (2, 1), (3, 2), (5, 2), (6, 4), (11, 4), (12, 8), (36, 8), (37, 16)])
+def test_z_run_of_a_batch(fake, cases, run):
+    """Cases of 16 columns by 16 planes on 296 resident thread blocks, one wave of single planes each
+    alone: single planes up to 1.8 waves, then two; 4, 8 and 16 planes as soon as their rules hold.  A case
+    with a run of its own keeps it."""
+    fake(f"""
+    ss = [box(128, 64, 16) for _ in range({cases})]
+    assert all(s.kernel() == (4, 1) for s in ss)
+    def runs():
+        b = aero.Batch(ss)
+        fake.fake_clear()
+        b.step(2)
+        got = [16 // int(l[2]) for l in log() if l[0] == "launch"]
+        assert len(got) == 4 * len(ss) and all(s.kernel()[0] == 4 for s in ss)
+        return got
+    assert set(runs()) == {{{run}}}
+    assert all(s.kernel() == (4, 1) for s in ss)
+    ss[0].set_kernel(4, 8)
+    assert set(runs()[:4]) == {{8}}
+    """)
