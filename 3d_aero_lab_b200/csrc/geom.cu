@@ -82,8 +82,9 @@ __device__ bool solid_at(const GeoDev& g, double x, double y, double z) {
     const double r = (double)v.env_R[k] + ((double)v.env_R[k + 1] - (double)v.env_R[k]) * (f - k);
     if (hypot(ay - v.y, z - v.z) < r) return true;
   }
-  // fuselage (AirGeom.inFus); no radius exceeds the larger of R0 and Re while noseP >= 0
-  if (x >= 0 && x <= a.fus_L && (ay <= 1.0001 * fmax(a.fus_R0, a.fus_Re) || a.fus_noseP < 0)) {
+  // fuselage (AirGeom.inFus); no radius exceeds the larger of R0 and Re while noseP >= 0 (radii count
+  // by their squares)
+  if (x >= 0 && x <= a.fus_L && (ay <= 1.0001 * fmax(fabs(a.fus_R0), fabs(a.fus_Re)) || a.fus_noseP < 0)) {
     const double R = fus_radius(a, x), dz = z - fus_center(a, x);
     if (ay * ay + dz * dz <= R * R) return true;
   }

@@ -24,6 +24,21 @@ def test_geometry_matches_oracle(aero, ref, typ, cells, delta):
         assert {3, 4, 5} <= set(np.unique(geo.t).tolist())
 
 
+@pytest.mark.parametrize("form", [dict(R0=-1, Re=-1, tailUp=-1), dict(R0=-1), dict(Re=-3), dict(Re=4), dict(R0=0),
+                                  dict(Re=0), dict(noseP=0), dict(noseP=-0.2), dict(noseP=3), dict(Ln=9), dict(Lt=-1)])
+def test_fuselages_of_every_form_match_oracle(aero, ref, form):
+    """The inside test leaves out points further from the symmetry plane than any radius: fuselages with
+    flared, pointed, bulging or formally negative ends (factors on the fighter's) give the oracle's cells."""
+    sh = aero.shape_of(aero.build_aircraft("fighter"))
+    g, og = aero.cfd_grid(sh, 30000), ref.grid(sh, 30000)
+    for k, f in form.items():
+        setattr(sh, "fus_" + k, getattr(sh, "fus_" + k) * f)
+    geo, o = aero.cfd_geom(sh, g, 2.0), ref.geom(sh, og, 2.0)
+    assert np.array_equal(geo.t, o.t) and np.array_equal(geo.phi, o.phi)
+    for d in range(4):
+        assert np.array_equal(geo.ap[d], o.ap[d]), d
+
+
 @pytest.mark.parametrize("typ,cells,delta", CASES[:4])
 def test_force_list_matches_oracle(aero, ref, typ, cells, delta):
     sh = aero.shape_of(aero.build_aircraft(typ))
