@@ -83,6 +83,36 @@ def test_stream_mode_equals_individual_steps(aero, n):
     b.dispose()
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kz", [0, 16])
+def test_first_order_batch_matches_the_single_cell_tile(aero, mode, kz):
+    """First order inside a batch - its own instances in the graph, the order of the arguments in the
+    persistent kernel - against the case alone, bit for bit, and against the single-cell tile, which
+    sums the same float32 terms in another order: the two tiles' 4e-6 after 20 iterations.  Two
+    cases keep second order, so that the batch mixes both."""
+    def cases(kernel):
+        out = [aero.Case(aircraft_type=c[0], cells=c[1], M=c[2], alpha=c[3], delta=c[4], kernel=kernel) for c in CASES]
+        for k, c in enumerate(out):
+            if kernel == 4:
+                c.solver.set_kernel(4, kz)
+            c.solver.set_opt(order=1 + k % 2)
+        return out
+
+    alone, tile, batched = cases(4), cases(2), cases(4)
+    b = aero.Batch([c.solver for c in batched])
+    b.set_mode(mode)
+    b.step(20)
+    b.sync()
+    for a, t, c in zip(alone, tile, batched):
+        a.solver.step(20)
+        t.solver.step(20)
+        A, T, B = (x.solver.read_array().astype(np.float64) for x in (a, t, c))
+        assert np.array_equal(A, B)
+        for v in range(5):
+            assert np.abs(T[v] - B[v]).max() < 4e-6 * np.abs(T[v]).max()
+    b.dispose()
+
+
 @pytest.mark.parametrize("scale", [0.1, 1, 4, 14])
 def test_automatic_z_runs_in_a_batch_leave_the_results(aero, scale):
     """Mode 1 over the paired tile: cases whose z run is automatic share a longer one (none, 4, 8 and
