@@ -123,6 +123,7 @@ cudaError_t dev_alloc_raw(void** p, size_t bytes) {
   } else {
     e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) return e;
   }
   std::lock_guard<std::mutex> lk(g_pool_mu);
   Pool* q = nullptr;

@@ -455,8 +455,8 @@ namespace {
 // a3d_solver_plane_ptr, only a wait for the device covers.
 cudaError_t wait_for_users(const a3d_solver* s) {
   cudaError_t e = s->st ? cudaStreamSynchronize(s->st) : cudaSuccess;
-  for (cudaStream_t c : s->cst)
-    if (c && e == cudaSuccess) e = cudaStreamSynchronize(c);
+  for (cudaStream_t c : s->cst)  // (after a step that failed half-way; else the solver's stream comes after them)
+    if (c && s->chunks_open && e == cudaSuccess) e = cudaStreamSynchronize(c);
   if (s->foreign && e == cudaSuccess) e = device_wait();
   return e;
 }
@@ -469,6 +469,7 @@ extern "C" int a3d_solver_destroy(a3d_solver* s) {
   const cudaError_t e = wait_for_users(s);
   if (e != cudaSuccess) {  // its memory and streams go to no other solver
     set_error("the solver's work could not be waited for: %s", cudaGetErrorString(e));
+    cudaGetLastError();  // (the next call's launches are not to report it)
     return A3D_ERR_CUDA;
   }
   dev_free(s->state);
@@ -551,6 +552,7 @@ int step_chunked(a3d_solver* s, int n, int K) {
     ke[c] = chunk_first(s, K, c + 1);
   }
   A3D_TRY(chunk_streams(s, K));  // (there already, unless the caller has set the chunks)
+  s->chunks_open = true;
   A3D_CUDA(cudaEventRecord(s->ev_fork, s->st));
   for (int c = 0; c < K; c++) A3D_CUDA(cudaStreamWaitEvent(s->cst[c], s->ev_fork, 0));
   bool first = true;
@@ -579,6 +581,7 @@ int step_chunked(a3d_solver* s, int n, int K) {
     s->it++;
   }
   for (int c = 0; c < K; c++) A3D_CUDA(cudaStreamWaitEvent(s->st, s->cev[c][1], 0));
+  s->chunks_open = false;
   return A3D_OK;
 }
 

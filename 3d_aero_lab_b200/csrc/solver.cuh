@@ -100,6 +100,7 @@ struct a3d_solver {
   cudaStream_t cst[a3d::kMaxChunks] = {};
   cudaEvent_t cev[a3d::kMaxChunks][2] = {};
   cudaEvent_t ev_fork = nullptr;
+  bool chunks_open = false;       // a chunk's stream may hold work that st does not come after
 };
 
 namespace a3d {

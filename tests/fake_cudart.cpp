@@ -30,6 +30,7 @@ size_t in_use = 0, idle[64] = {};
 long next_handle = 16, pools = 0;
 thread_local int device = 0;
 thread_local Call pushed;
+thread_local cudaError_t last = cudaSuccess;
 
 cudaError_t log(const char* f, const char* fmt = "", ...) {
   std::lock_guard<std::recursive_mutex> lk(mu);
@@ -41,7 +42,8 @@ cudaError_t log(const char* f, const char* fmt = "", ...) {
   text += std::string(f) + " " + b + "\n";
   auto it = fail.find(f);
   if (it == fail.end() || it->second.calls-- != 1) return cudaSuccess;
-  return (cudaError_t)it->second.status;
+  last = (cudaError_t)it->second.status;
+  return last;
 }
 
 template <typename T>
@@ -150,7 +152,11 @@ cudaError_t cudaDeviceSynchronize() {
   LOGGED("cudaDeviceSynchronize");
   return knob["capturing"] ? cudaErrorStreamCaptureUnsupported : cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = last;
+  last = cudaSuccess;
+  return e;
+}
 
 // ---- memory
 cudaError_t cudaMalloc(void** p, size_t n) { LOGGED("cudaMalloc", "%zu", n); return take(p, n, -1); }

@@ -129,8 +129,21 @@ def test_destruction_waits_for_its_own_streams_and_spoils_no_capture(fake):
     L = log()
     freed = [i for i, l in enumerate(L) if l[0] in ("cudaFree", "cudaFreeAsync")]
     waited = {l[1] for l in L[:freed[0]] if l[0] == "cudaStreamSynchronize"}
-    assert own in waited and len(waited) == 4            # its own and the chunks'
+    assert waited == {own}                                           # which comes after the chunks'
     assert not [l for l in L if l[0] == "cudaMalloc"]                # nobody else had its address
+    c = box(6, 4, 9)
+    c.set_kernel(4, 2)
+    c.set_chunks(3)
+    c.step(1)
+    fake.fake_fail(b"launch", 1, 5)                                  # a step that fails half-way
+    assert lib.a3d_solver_step(c._h, 1) != 0
+    own = str(c.stream)
+    fake.fake_clear()
+    c.dispose()
+    L = log()
+    freed = [i for i, l in enumerate(L) if l[0] in ("cudaFree", "cudaFreeAsync")]
+    waited = {l[1] for l in L[:freed[0]] if l[0] == "cudaStreamSynchronize"}
+    assert own in waited and len(waited) == 4                        # the chunks' own too
     b.plane_ptr(0, 0, 0)                                             # b's address is out: the device is waited for
     fake.fake_clear()
     b.dispose()
