@@ -12,11 +12,13 @@ namespace a3d {
 void set_error(const char* fmt, ...);
 void clear_error();
 
-// CUDA call wrapper: on failure record "<call> @ file:line: <cuda message>" and return.
+// CUDA call wrapper: on failure record "<call> @ file:line: <cuda message>" and return.  The runtime's
+// own record of the failure is cleared: the check after a later call's launch would report it.
 #define A3D_CUDA(call)                                                                      \
   do {                                                                                      \
     cudaError_t e_ = (call);                                                                \
     if (e_ != cudaSuccess) {                                                                \
+      cudaGetLastError();                                                                   \
       ::a3d::set_error("%s @ %s:%d: %s", #call, __FILE__, __LINE__, cudaGetErrorString(e_)); \
       return (e_ == cudaErrorMemoryAllocation) ? A3D_ERR_NOMEM : A3D_ERR_CUDA;              \
     }                                                                                       \

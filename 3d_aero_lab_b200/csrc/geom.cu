@@ -412,10 +412,8 @@ int geom_build_device(const a3d_shape& shape, const GridDev& gd, double h, doubl
     else if ((e = cudaGetLastError()) != cudaSuccess) fail(e, "geometry launch");
     if (counts) { counts[0] = (int64_t)hc[0]; counts[1] = (int64_t)hc[1]; }
   }
-  cudaFreeAsync(d_cnt, st);
-  cudaFreeAsync(mark, st);
-  cudaFreeAsync(cin, st);
-  cudaFreeAsync(d_shape, st);
+  for (void* p : {(void*)d_cnt, (void*)mark, (void*)cin, (void*)d_shape})
+    if (p) cudaFreeAsync(p, st);
   cudaStreamSynchronize(st);
   return rc;
 }

@@ -130,6 +130,7 @@ cudaError_t dev_alloc_raw(void** p, size_t bytes) {
   if (current_pool(&q) != cudaSuccess) return e;
   if (e == cudaSuccess && large) q->large.insert(*p);
   if (e != cudaSuccess && !large) q->blocks--;
+  if (e != cudaSuccess) cudaGetLastError();  // (reported by the caller; not by its next launch's check)
   return e;
 }
 
@@ -208,7 +209,9 @@ cudaError_t temp_alloc_raw(void** p, size_t bytes, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     pool = q->pool;
   }
-  return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, st);
+  const cudaError_t e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, st);
+  if (e != cudaSuccess) cudaGetLastError();  // (as in dev_alloc)
+  return e;
 }
 
 // (asked once for each pair: cudaMemPoolSetAccess is no call for every halo exchange)

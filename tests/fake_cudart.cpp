@@ -57,7 +57,7 @@ cudaError_t take(void** p, size_t bytes, int pool) {
   const size_t reuse = pool >= 0 && bytes <= idle[pool] ? bytes : 0;  // (idle memory is one piece)
   size_t held = in_use;
   for (size_t i : idle) held += i;
-  if (held + bytes - reuse > (size_t)knob["limit"]) return cudaErrorMemoryAllocation;
+  if (held + bytes - reuse > (size_t)knob["limit"]) return last = cudaErrorMemoryAllocation;
   if (pool >= 0) idle[pool] -= reuse;
   in_use += bytes;
   *p = calloc(1, bytes + 256);
@@ -186,7 +186,9 @@ cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t pool, cuda
   LOGGED("cudaMallocFromPoolAsync", "%ld %zu", (long)st, n);
   return take(p, n, (int)(long)pool);
 }
-cudaError_t cudaFreeAsync(void* p, cudaStream_t st) { LOGGED("cudaFreeAsync", "%ld %p", (long)st, p); return give(p); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t st) {
+  if (!p) return last = cudaErrorInvalidValue;  // (unlike cudaFree)
+  LOGGED("cudaFreeAsync", "%ld %p", (long)st, p); return give(p); }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
   LOGGED("cudaMemcpy", "%d", (int)k);
   memcpy(d, s, n);

@@ -266,3 +266,30 @@ def test_z_run_of_a_batch(fake, cases, run):
     ss[0].set_kernel(4, 8)
     assert set(runs()[:4]) == {{8}}
     """)
+
+
+@pytest.mark.parametrize("size", ["60, 40, 50", "600, 200, 40"])  # the state in the pool, from cudaMalloc
+@pytest.mark.parametrize("make", ["box({})", "aero.CfdGPU(box_grid({}), shape=shape)"])
+def test_a_case_without_memory_fails_alone(fake, size, make):
+    """The call that found no memory says so and leaves nothing behind: neither blocks, nor a CUDA
+    error that another solver's next launch would report."""
+    fake(f"""
+    shape = aero.shape_of(aero.build_aircraft("fighter"))
+    def box_grid(*n):
+        return cfd.Grid(*[np.arange(k + 1, dtype=np.float64) for k in n])
+    s = box(6, 4, 9)
+    live = fake.fake_live()
+    for limit in (10**4, 10**6, 3 * 10**6, 5 * 10**6, 12 * 10**6, 10**8, 3 * 10**8):
+        fake.fake_set(b"limit", limit)
+        try:
+            x = {make.format(size)}
+        except aero.AeroError as e:
+            assert e.status == 3, e
+        else:
+            x.dispose()
+            del x
+        s.step(2)
+        s.mach_max()
+        assert fake.fake_live() == live
+    fake.fake_set(b"limit", 1 << 50)
+    """)
