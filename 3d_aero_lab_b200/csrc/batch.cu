@@ -237,8 +237,9 @@ std::vector<double> signature(const a3d_solver* s) {
 }
 
 // Mode 1: the z run of the cases whose own is automatic (paired tile only, whose results do not
-// depend on the run): *kz, or where that is 0 their own, but at least *least.  A case's own run is short enough to fill the chip alone;
-// beside others it need not be, and each run costs four planes read and a z face formed twice.
+// depend on the run): *kz, or where that is 0 their own, but at least *least.  A case's own run is
+// short enough to fill the chip alone; beside others it need not be, and each run costs four planes
+// read and a z face formed twice.
 // So: 16 planes where all cases together still launch two waves of CTAs, else 8 or 4 planes where
 // that makes 1.2 waves.  Measured (us per iteration; own runs, 4, 8, 16 planes): 24 cases, 5.1M
 // cells 475, 408, 372, 369 (3.4 waves at 16); 5 cases, 4.4M 322, 301, 281, 280 (2.4); 8 cases, 2.5M

@@ -43,8 +43,9 @@ int use_device(int device) {
 // cudaMalloc, cudaFree and the default pool (which gives its memory back at every
 // synchronisation) map and unmap device memory: 0.2 to 6 ms a call, more than the work of a
 // case's setup (1M cells: 12 ms with a dozen of them, 0.3 ms of kernels) or of sampling 20,000
-// points.  The library therefore has a pool of its own on each device: 2 us a call.  It keeps at
-// most kPoolKeep bytes that nothing uses, and nothing at all once the last block is freed.
+// points.  The library therefore has a pool of its own on each device: 2 us a call.  Memory that
+// nothing uses stays while the pool's whole, used and unused, is below kPoolKeep bytes, and not at
+// all once the last block is freed (the next case then pays as without the pool).
 // Blocks beyond kPoolBlock, of which a pool could keep none, come from cudaMalloc as before (growing
 // the pool by gigabytes takes longer: 120M cells' setup 0.12 s instead of 0.10).
 namespace {

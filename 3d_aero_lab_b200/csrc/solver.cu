@@ -858,7 +858,7 @@ int auto_run_tma(long columns, int NZ, int resident) {
 // us per iteration, picked / 2 planes: 268k 32.0 / 38.6 (3 planes), 522k 46.2 / 52.2 (5), 675k 53.5 /
 // 59.8 (6); single planes up to one wave: 31k 17.9 against 24.6.
 int auto_run_pair(long columns, int NZ, long cells, int resident) {
-  if (cells >= kChunkCells) return (int)std::clamp(std::lround(columns * NZ / (2.5 * resident)), 2L, 32L);
+  if (cells >= kChunkCells) return (int)std::clamp(std::lround(columns * NZ / (2.5 * resident)), 3L, 32L);
   int best = 1;
   double least = INFINITY;
   for (int kz = 1; kz <= std::min(NZ, 16); kz++) {

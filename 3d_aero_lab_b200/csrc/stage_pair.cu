@@ -10,7 +10,8 @@ namespace {
 
 using namespace pair;
 
-// At most 128 registers: two CTAs (16 warps) per SM.  MODE 0: all planes of a lone case, dependent on
+// At most 128 registers: two CTAs (16 warps) per SM (one of the twelve spills, 4 bytes: stage 2 of a lone
+// first-order case).  MODE 0: all planes of a lone case, dependent on
 // the launch before; 1: planes [a.kb, a.ke) (a z chunk, a slab's own planes, a case of a batch); 2: the
 // same with the halo push of a z slab.
 template <bool STAGE2, int MODE, int ORDER>

@@ -13,9 +13,9 @@
 // loop is kept short and what only cells beside a body need - apertures, the wall-pressure
 // source, baffles - stands behind one test of the pair's codes.  9009 warp instructions per plane
 // of a tile in stage 1 (9712 with the apertures carried through shared memory and the wall term
-// formed for every cell); fighter 4.13M cells 17.05 -> 18.7 G cell-updates/s, airliner 120M 19.9 ->
-// 22.3 (22.6 with the order of the scheme a constant).  The loop must also fit the instruction caches: unrolled by two planes, which removes the
-// 42 register moves a plane and pair, it is 37 KB long and measured 18.0 at 120M.
+// formed for every cell): airliner 120M 19.9 -> 22.3 G cell-updates/s.  The loop must also fit the
+// instruction caches: unrolled by two planes, which removes the 42 register moves a plane and pair,
+// it is 37 KB long and measured 18.0 at 120M.
 //
 // The planes arrive through a 4-deep ring of shared-memory slots filled by
 // `cp.async.bulk.tensor` (one 40 x 20 x 5-component state box and one 64 x 20 code box per
@@ -379,13 +379,13 @@ __device__ __forceinline__ void store_pair(const StageArgs& a, float* __restrict
 // slab's own planes, one z chunk of a pipelined step, a case of a batch), ordered by events;
 // without it the launch is a lone case's, dependent on the one before it.
 // ORDER: 1 or 2 where the order of the scheme is the kernel's, 0 where it comes with the arguments.
-// First order needs no slopes, which were formed and multiplied by 0: us per iteration at first order
-// with the order in the arguments / in the kernel 31k 16.8 / 14.6, 0.39M 42.8 / 37.0, 4.1M 227 / 181,
-// 120M 5398 / 4182 (28.7 G cell-updates/s); at second order, by the constant alone, 120M 5397 / 5326.  PUSH: stores also go to the
-// neighbour slab that keeps the plane as a halo plane.
+// First order needs no slopes, which were formed and multiplied by 0: us per iteration with the order
+// in the arguments / in the kernel 31k 16.8 / 14.6, 4.1M 227 / 181; at second order 120M 5397 / 5326.
+// PUSH: stores also go to the neighbour slab that keeps the plane as a halo plane.
 template <bool STAGE2, bool PERSISTENT, bool RANGE = false, bool PUSH = false, int ORDER = 0>
-__device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const StageArgs& a, const float* __restrict__ Bp, float* __restrict__ Outp, int bx, int by, int bz,
-                                           int kz) {
+__device__ __forceinline__ bool stage_tile(PairSmem& S, const Maps& maps, const StageArgs& a,
+                                           const float* __restrict__ Bp, float* __restrict__ Outp, int bx, int by,
+                                           int bz, int kz) {
   const int t = threadIdx.x, tx2 = t & 15, ty = t >> 4;
   const int i0 = bx * TX, j0 = by * TY;
   const int x0 = i0 + 2 * tx2, j = j0 + ty;

@@ -247,7 +247,7 @@ int a3d_solver_plane_ptr(a3d_solver* s, int32_t which, int32_t c, int32_t k, voi
  * and upper neighbours (either may be NULL) keep as halo planes into the neighbours' buffers,
  * peer stores across devices.  Afterwards s advances only by a3d_solver_stage; call
  * a3d_solver_sync_neighbors on every slab after every stage of all slabs, so that each slab's
- * next stage waits for its neighbours' stores.  Stage kernels 0 and 2.                   */
+ * next stage waits for its neighbours' stores.  Stage kernels 0, 2 and 4.                */
 int a3d_solver_set_neighbors(a3d_solver* s, a3d_solver* lo, a3d_solver* hi);
 int a3d_solver_sync_neighbors(a3d_solver* s);
 /* Sum of squared density changes and cell count behind the last a3d_solver_residual.     */
@@ -288,8 +288,8 @@ int a3d_batch_tune(a3d_batch* b, int32_t trial_iters, int32_t* best_kz, int32_t*
 /* No counterpart in the reference (its controller steps one case per animation frame).  A
  * scheduler thread admits requests in arrival order while the estimated device memory of all
  * resident cases fits `hbm_budget_bytes` and fewer than `max_active` run; every round advances
- * all active cases by `chunk_iters` iterations in one batch (one persistent launch per RK
- * stage), then checks each case's FP64 density residual (every fluid cell) against its first
+ * all active cases by `chunk_iters` iterations in one batch (every case's own launches, in
+ * one CUDA graph), then checks each case's FP64 density residual (every fluid cell) against its first
  * value.  A case finishes when the ratio is <= residual_drop or after max_iters iterations;
  * its forces and Trefftz drag are computed on the device and it leaves the batch at once.
  * With warm_start, finished cases stay resident keyed by `geometry_key` and a later request

@@ -1,8 +1,8 @@
 """Batched persistent-kernel runs: every case bit-identical to the same case stepped alone, for
-both batch tiles (kernel 2: the TMA tile, kernel 4: the paired-cell tile).  The tiles form the
-first z face of a run in their prologue, where the compiler may round one operation
+both batch tiles (kernel 2: the TMA tile, kernel 4: the paired-cell tile).  The TMA tile forms the
+first z face of a run in its prologue, where the compiler may round one operation
 differently, so a case is bit-identical at equal run length and agrees to float32 rounding
-across run lengths."""
+across run lengths; the paired tile's cases are bit-identical across run lengths too."""
 import threading
 
 import numpy as np

@@ -1,8 +1,8 @@
 """One case on z slabs (split.py) against the same case unsplit, on one GPU.
 
 With the halo planes exchanged after each stage, a slab's own planes see the numbers of the
-unsplit solve.  The per-cell kernel and the z-marching TMA tiles (single-cell and paired) with
-slab boundaries aligned to their z runs give the same state bit for bit.  Unaligned, a tile
+unsplit solve.  The per-cell kernel, the paired tile and the single-cell tile with slab
+boundaries aligned to its z runs give the same state bit for bit.  Unaligned, the single-cell tile
 differs only where a z run starts elsewhere, within the 4e-6 of its prologue rounding.  The FP64 reductions sum
 the same terms in another order.
 """
