@@ -153,6 +153,19 @@ def test_destruction_waits_for_its_own_streams_and_spoils_no_capture(fake):
     """)
 
 
+def test_a_solver_can_be_dropped_when_memory_has_run_out(fake):
+    """Whose address a caller holds: there is no byte left to wait for the device with."""
+    fake("""
+    s = box(6, 4, 9)
+    s.plane_ptr(0, 0, 0)
+    fake.fake_set(b"limit", 0)
+    assert lib.a3d_solver_destroy(s._h) == 0
+    s._h = C.c_void_p()
+    assert fake.fake_live() == 0
+    assert [l for l in log() if l[0] == "cudaDeviceSynchronize"]
+    """)
+
+
 def test_memory_of_a_solver_that_could_not_be_waited_for_is_not_recycled(fake):
     fake("""
     s = box(6, 4, 9)
