@@ -236,7 +236,7 @@ def test_first_order_tile_matches_the_single_cell_tile(aero, cells, kz, chunks):
 
 @pytest.mark.parametrize("kernel", [2, 4])
 def test_bounded_wait_runs_out_reports_timeout_and_recovers(aero, kernel):
-    """The TMA tiles' bounded waits (SURVEY failure detection): with the wait limit at 0 every wait
+    """The TMA tiles' bounded waits: with the wait limit at 0 every wait
     for a plane copy gives up at once; the kernel drains its copies in flight, flags the solver
     and leaves, nothing faults, and the host gets A3D_ERR_TIMEOUT once.  With the default limit
     back and the state reset, the same solver steps exactly like a fresh one."""
